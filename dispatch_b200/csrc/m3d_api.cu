@@ -1142,6 +1142,33 @@ int m3d_upstream_boundary(const m3d_slab_t *slab, void *work, int mode, const vo
 
 namespace {
 
+int sm_count();   // m3d_stateq_api.inc
+
+// 72 KB of tables in shared memory for a lane kernel
+int lane_attr(const void *kernel) {
+  CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(2 * QLG_NTAB * sizeof(float))));
+  return M3D_OK;
+}
+
+// a zeroed counter of the units handed out by the next launch
+int unit_counter(int **next) {
+  void *p;
+  TRY(scratch(28, sizeof(int), &p));
+  CUDA_TRY(cudaMemsetAsync(p, 0, sizeof(int), g_ctx.stream));
+  *next = (int *)p;
+  return M3D_OK;
+}
+
+// the directions of a call on the device
+int stage_directions(const double *vec, int nray, const double **d_vr) {
+  void *p;
+  TRY(scratch(26, sizeof(double) * 3 * nray, &p));
+  CUDA_TRY(cudaMemcpyAsync(p, vec, sizeof(double) * 3 * nray, cudaMemcpyHostToDevice, g_ctx.stream));
+  *d_vr = (const double *)p;
+  return M3D_OK;
+}
+
 // The atmosphere, line lists and window of the LTE pass on the device
 struct SynthIn {
   AtmosDev A;
@@ -1153,12 +1180,9 @@ struct SynthIn {
   const double *dnu = nullptr, *dllam = nullptr;
   int nf = 0;
   size_t ncell = 0;
-  // a batch of nwin windows of nf frequencies (nu, llam of nwin nf), each with its grid,
-  // for nray directions d_vr (3 each) in one launch
+  // a batch of nwin windows of nf frequencies (nu, llam of nwin nf), each with its grid
   int nwin = 1;
   const GridArgs *d_Gw = nullptr;
-  int nray = 1;
-  const double *d_vr = nullptr;
 };
 
 int stage_synthesis(Staging &st, const m3d_atmos_t *atm, int nf, const double *nu, const double *llam, bool fp64,
@@ -1219,86 +1243,101 @@ int stage_synthesis(Staging &st, const m3d_atmos_t *atm, int nf, const double *n
   return M3D_OK;
 }
 
-// Line opacity + transfer units of every cell for direction v: (chi, S) of the
-// window, frequency fastest per cell.  FP32: the lane-per-cell kernel for windows of
-// 32 frequencies, the warp-per-cell kernel otherwise; FP64: the plain FP64 kernel.
-int launch_opacity(SynthIn &in, const double *v, bool fp64, void *dchi, void *dS) {
+// The lane kernel's form for a window of nf frequencies: NF registers a lane, P lanes a
+// cell.  Windows wider than 64 give a cell 2 to 16 lanes of 64 registers; below 8
+// frequencies the warp-per-cell kernel takes over (NF = 0).
+struct LaneForm { int NF, P; };
+LaneForm lane_form(int nf) {
+  if (nf < 8) return {0, 32};
+  if (nf <= 64) return {nf <= 16 ? 16 : nf <= 32 ? 32 : nf <= 48 ? 48 : 64, 1};
+  int P = 2;
+  while (64 * P < nf) P *= 2;
+  return {64, P};
+}
+
+// Rays of one opacity launch.  A launch holds 148 x 24 warps at a time; eight times as
+// many keep the last, partly filled round of warps to a few percent of the launch, and
+// more would only cost memory.  The units of the launch's rays stay within 512 MB.
+int rays_per_launch(size_t ncell, int nf, int nray, size_t esz) {
+  const LaneForm lf = lane_form(nf);
+  const size_t warps = std::max<size_t>(1, ncell * lf.P / 32);
+  size_t r = (148 * 24 * 8 + warps - 1) / warps;
+  r = std::min(r, ((size_t)512 << 20) / std::max<size_t>(1, 2 * esz * nf * ncell));
+  r = std::max<size_t>(1, std::min<size_t>(r, nray));
+  const size_t groups = (nray + r - 1) / r;      // as even as they come
+  return (int)((nray + groups - 1) / groups);
+}
+
+// Line opacity + transfer units of every cell for nray directions (d_vr on the device,
+// v their host copy): (chi, S) of the window, frequency fastest per cell, ray after ray.
+// FP32: the lane-per-cell kernel; the warp-per-cell kernel for windows below 8
+// frequencies, and for lists with reach_in unless the window has 32 (one ray a launch
+// either way).  FP64: the plain FP64 kernel.
+int launch_opacity(SynthIn &in, const double *v, const double *d_vr, int nray, bool fp64, void *dchi, void *dS) {
   const int nf = in.nf;
   const size_t ncell = in.ncell;
   const int block = 256, warps = block / 32;
-  const bool batch = in.nwin > 1;
+  const bool wins = in.nwin > 1;
+  const GridArgs *no_gw = nullptr;
   if (fp64) {
-    int grid = (int)((ncell * in.nwin * (batch ? in.nray : 1) + block - 1) / block);
-    if (grid > 148 * 8) grid = 148 * 8;
-    if (batch)
-      LAUNCH_S(M3D_STAGE_OPACITY, (k_lte_opacity_units_f64<32, true>), grid, block, 0, in.A, in.G, in.dnu, 0.0, 0.0,
-               0.0, (double *)dchi, (double *)dS, (const double2 *)g_ctx.d_tab64, in.d_Gw, in.nwin, in.d_vr, in.nray);
+    const size_t want = (ncell * in.nwin * nray + block - 1) / block;
+    const int grid = (int)std::min<size_t>(want, 148 * 8);
+    if (wins)
+      LAUNCH_S(M3D_STAGE_OPACITY, (k_lte_opacity_units_f64<32, true>), grid, block, 0, in.A, in.G, in.dnu,
+               (double *)dchi, (double *)dS, (const double2 *)g_ctx.d_tab64, in.d_Gw, in.nwin, d_vr, nray);
     else if (nf == 32)
-      LAUNCH_S(M3D_STAGE_OPACITY, k_lte_opacity_units_f64<32>, grid, block, 0, in.A, in.G, in.dnu, v[0], v[1], v[2],
-               (double *)dchi, (double *)dS, (const double2 *)g_ctx.d_tab64, (const GridArgs *)nullptr, 1,
-               (const double *)nullptr, 1);
+      LAUNCH_S(M3D_STAGE_OPACITY, k_lte_opacity_units_f64<32>, grid, block, 0, in.A, in.G, in.dnu, (double *)dchi,
+               (double *)dS, (const double2 *)g_ctx.d_tab64, no_gw, 1, d_vr, nray);
     else
-      LAUNCH_S(M3D_STAGE_OPACITY, k_lte_opacity_units_f64<0>, grid, block, 0, in.A, in.G, in.dnu, v[0], v[1], v[2],
-               (double *)dchi, (double *)dS, (const double2 *)g_ctx.d_tab64, (const GridArgs *)nullptr, 1,
-               (const double *)nullptr, 1);
+      LAUNCH_S(M3D_STAGE_OPACITY, k_lte_opacity_units_f64<0>, grid, block, 0, in.A, in.G, in.dnu, (double *)dchi,
+               (double *)dS, (const double2 *)g_ctx.d_tab64, no_gw, 1, d_vr, nray);
     return M3D_OK;
   }
-  const bool lane32 = nf == 32;
-  const size_t smem_op = lane32 ? 2 * QLG_NTAB * sizeof(float)
-                                : (2 * QLG_NTAB + (size_t)warps * 4 * nf) * sizeof(float);
-  {
-    thread_local size_t attr[2] = {0, 0};
-    const int which = lane32 ? 1 : 0;
-    if (attr[which] < smem_op) {
-      if (lane32) {
-        CUDA_TRY(cudaFuncSetAttribute((const void *)k_lte_opacity_units_lane<32, float, false>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_op));
-        CUDA_TRY(cudaFuncSetAttribute((const void *)k_lte_opacity_units_lane<32, float, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_op));
-        CUDA_TRY(cudaFuncSetAttribute((const void *)k_lte_opacity_units_lane<32, float, false, false, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_op));
-      } else {
-        CUDA_TRY(cudaFuncSetAttribute((const void *)k_lte_opacity_units<float>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_op));
-      }
-      attr[which] = smem_op;
-    }
-  }
   if (in.reach) {
+    if (nray != 1) return fail(M3D_EINVAL, "launch_opacity: one ray at a time with reach_in");
     CUDA_TRY(cudaMemsetAsync(in.d_vmax, 0, sizeof(unsigned), g_ctx.stream));
     LAUNCH(k_vproj_absmax, grid_for(ncell), 256, 0, in.A, v[0], v[1], v[2], in.d_vmax);
     for (int k = 0; k < in.A.nspecies; k++)
       LAUNCH(k_select_lines, 1, 32, 0, in.sp[k].L, in.dllam, nf, (const unsigned *)in.d_vmax, in.d_sel[k],
              in.d_nsel[k]);
   }
-  if (lane32) {
-    // lane kernel: one warp per 32 cells (of one window), grid-stride over warps.  One
-    // block of 24 warps per SM: the QLG tables are staged once per SM (72 KB), where
-    // three blocks of 8 warps (the same occupancy) held three copies and left L1 almost
-    // no room for the line list and the cells' fields; 3.55 -> 4.08 Gpt*nu*ray/s on the
-    // 240^3 configuration
-    const size_t nvc = (ncell + 31) / 32 * 32 * (size_t)in.nwin * (batch ? in.nray : 1);
-    const int lblock = 768;
-    int lgrid = (int)((nvc + lblock - 1) / lblock);
-    if (lgrid > 148 * 8) lgrid = 148 * 8;
-    if (batch)
-      LAUNCH_S(M3D_STAGE_OPACITY, (k_lte_opacity_units_lane<32, float, false, false, true>), lgrid, lblock, smem_op,
-               in.A, in.G, in.dnu, 0.0, 0.0, 0.0, (float *)dchi, (float *)dS, g_ctx.d_tab, in.d_Gw, in.nwin, in.d_vr,
-               in.nray);
-    else if (in.reach)
-      LAUNCH_S(M3D_STAGE_OPACITY, (k_lte_opacity_units_lane<32, float, true>), lgrid, lblock, smem_op, in.A, in.G,
-               in.dnu, v[0], v[1], v[2], (float *)dchi, (float *)dS, g_ctx.d_tab, (const GridArgs *)nullptr, 1,
-               (const double *)nullptr, 1);
-    else
-      LAUNCH_S(M3D_STAGE_OPACITY, (k_lte_opacity_units_lane<32, float, false>), lgrid, lblock, smem_op, in.A, in.G,
-               in.dnu, v[0], v[1], v[2], (float *)dchi, (float *)dS, g_ctx.d_tab, (const GridArgs *)nullptr, 1,
-               (const double *)nullptr, 1);
-  } else {
-    int ogrid = (int)((ncell + warps - 1) / warps);
-    if (ogrid > 148 * 16) ogrid = 148 * 16;
-    LAUNCH_S(M3D_STAGE_OPACITY, k_lte_opacity_units<float>, ogrid, block, smem_op, in.A, in.G, in.dnu, v[0], v[1],
-             v[2], (float *)dchi, (float *)dS, g_ctx.d_tab);
+  const LaneForm lf = lane_form(nf);
+  if (lf.NF == 0 || (in.reach && nf != 32)) {
+    const size_t smem = (2 * QLG_NTAB + (size_t)warps * 4 * nf) * sizeof(float);
+    thread_local size_t attr = 0;
+    if (attr < smem) {
+      CUDA_TRY(cudaFuncSetAttribute((const void *)k_lte_opacity_units, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)smem));
+      attr = smem;
+    }
+    const int grid = (int)std::min<size_t>((ncell + warps - 1) / warps, 148 * 16);
+    for (int r = 0; r < nray; r++)
+      LAUNCH_S(M3D_STAGE_OPACITY, k_lte_opacity_units, grid, block, smem, in.A, in.G, in.dnu, v[3 * r], v[3 * r + 1],
+               v[3 * r + 2], (float *)dchi + (size_t)nf * ncell * r, (float *)dS + (size_t)nf * ncell * r,
+               g_ctx.d_tab);
+    return M3D_OK;
   }
+  // lane kernel: one block per SM, so the QLG tables are staged once per SM (72 KB)
+  // and L1 keeps room for the line list and the cells' fields (three blocks of 8 warps
+  // with a copy each: 3.55 against 4.08 Gpt*nu*ray/s on 240^3)
+  using LaneKernel = void (*)(AtmosDev, GridArgs, const double *, float *, float *, const float2 *, const GridArgs *,
+                              int, const double *, int, int, int *);
+  LaneKernel k;
+  if (lf.P > 1) k = k_lte_opacity_units_lane<64, false, false, false, false, true>;
+  else if (wins) k = k_lte_opacity_units_lane<32, false, false, true>;
+  else if (nf == 32 && in.reach) k = k_lte_opacity_units_lane<32, true>;
+  else if (nf == 32) k = k_lte_opacity_units_lane<32, false>;
+  else if (lf.NF == 16) k = k_lte_opacity_units_lane<16, false, false, false, true>;
+  else if (lf.NF == 32) k = k_lte_opacity_units_lane<32, false, false, false, true>;
+  else if (lf.NF == 48) k = k_lte_opacity_units_lane<48, false, false, false, true>;
+  else k = k_lte_opacity_units_lane<64, false, false, false, true>;
+  TRY(lane_attr((const void *)k));
+  int *next;
+  TRY(unit_counter(&next));
+  const size_t cw = 32 / lf.P, units = (ncell * nray + cw - 1) / cw * in.nwin;
+  const int grid = (int)std::min<size_t>(units, (size_t)sm_count());
+  LAUNCH_S(M3D_STAGE_OPACITY, k, grid, lane_threads(lf.NF), 2 * QLG_NTAB * sizeof(float), in.A, in.G, in.dnu,
+           (float *)dchi, (float *)dS, g_ctx.d_tab, in.d_Gw, in.nwin, d_vr, nray, lf.P, next);
   return M3D_OK;
 }
 
@@ -1339,7 +1378,9 @@ int m3d_lte_transfer_units(const m3d_atmos_t *atm, int nf, const double *nu, con
     TRY(st.map((float *)S, n, false, true, &b));
     dchi = a; dS = b;
   }
-  TRY(launch_opacity(in, vec, fp64, dchi, dS));
+  const double *d_vr;
+  TRY(stage_directions(vec, 1, &d_vr));
+  TRY(launch_opacity(in, vec, d_vr, 1, fp64, dchi, dS));
   return st.finish();
 }
 
@@ -1410,20 +1451,15 @@ int lte_synthesis_impl(const m3d_atmos_t *atm, int nwin, int nf_win, const doubl
                         (float)atm->tol, 0.0f);
       if (!(gw[w].dllam > 0)) return fail(M3D_EINVAL, "%s: window %d: log(lambda) must be ascending", who, w);
     }
-    void *dgw, *dvr;
+    void *dgw;
     TRY(scratch(25, sizeof(GridArgs) * gw.size(), &dgw));
     CUDA_TRY(cudaMemcpyAsync(dgw, gw.data(), sizeof(GridArgs) * gw.size(), cudaMemcpyHostToDevice, g_ctx.stream));
-    TRY(scratch(26, sizeof(double) * 3 * nray, &dvr));
-    CUDA_TRY(cudaMemcpyAsync(dvr, vec, sizeof(double) * 3 * nray, cudaMemcpyHostToDevice, g_ctx.stream));
     in.nf = nf_win;
     in.nwin = nwin;
     in.d_Gw = (const GridArgs *)dgw;
-    in.nray = nray;
-    in.d_vr = (const double *)dvr;
   }
-  // a batch holds every ray's transfer units at once (the opacity of all of them is
-  // one launch); a single window one ray's
-  const size_t nray_units = nwin > 1 ? (size_t)nray : 1;
+  const double *d_vr;
+  TRY(stage_directions(vec, nray, &d_vr));
 
   // rotation table of every global plane, per ray; slab starts
   // A single column is a plane-parallel atmosphere: radiative_transfer applies no
@@ -1453,11 +1489,20 @@ int lte_synthesis_impl(const m3d_atmos_t *atm, int nwin, int nf_win, const doubl
   CUDA_TRY(cudaMemcpyAsync(drot, rotc.data(), sizeof(RotCol) * rotc.size(), cudaMemcpyHostToDevice, g_ctx.stream));
   CUDA_TRY(cudaMemcpyAsync(dz0, z0.data(), sizeof(int) * z0.size(), cudaMemcpyHostToDevice, g_ctx.stream));
 
-  // transfer units of the whole column (one ray at a time) and the emergent planes
+  // transfer units of the whole column for a group of rays, and the emergent planes.
+  // A window batch holds every ray's units; so does a single window of few cells, and
+  // larger ones as many rays as fill the GPU (one, where they do not fit)
   const size_t esz = fp64 ? sizeof(double) : sizeof(float);
+  int group = nwin > 1 ? nray : (in.reach ? 1 : rays_per_launch(in.ncell, nf, nray, esz));
+  group = std::min(group, 32768);  // the grid limit of the launches below
   void *dchi, *dS, *dtop;
-  TRY(scratch(7, esz * plane * nz * nray_units, &dchi));
-  TRY(scratch(8, esz * plane * nz * nray_units, &dS));
+  if (nwin == 1 && group > 1 &&
+      (scratch(7, esz * plane * nz * group, &dchi) != M3D_OK || scratch(8, esz * plane * nz * group, &dS) != M3D_OK)) {
+    cudaGetLastError();
+    group = 1;
+  }
+  TRY(scratch(7, esz * plane * nz * group, &dchi));
+  TRY(scratch(8, esz * plane * nz * group, &dS));
   void *dtop_user = nullptr;
   if (i_top) {
     if (fp64) { double *p; TRY(st.map((double *)i_top, plane * nray, false, true, &p)); dtop_user = p; }
@@ -1466,16 +1511,32 @@ int lte_synthesis_impl(const m3d_atmos_t *atm, int nwin, int nf_win, const doubl
   } else {
     TRY(scratch(9, esz * plane * nray, &dtop));
   }
-  float *die;
+  float *die, *dflux;
   TRY(st.map(ie, (size_t)nf * nray, false, true, &die));
+  TRY(st.map(flux, (size_t)nf, false, true, &dflux));
 
   const float dtmax = -(float)atm->maser_dtau_max, Imax = (float)atm->maser_Inu_max;
   const PchipConst pc = pchip_const((float)atm->ds_code[2]);
 
-  // partial sums of the intensity reduction
-  const int kParts = 148;
+  // per ray: the solver's constants and the flux weight
+  std::vector<unsigned char> hray((sizeof(QuadConst) + sizeof(float)) * nray);
+  QuadConst *hqc = (QuadConst *)hray.data();
+  float *hw = (float *)(hqc + nray);
+  for (int r = 0; r < nray; r++) {
+    hqc[r] = quad_const(atm->ds_cm[2], vec[3 * r + 2]);
+    hw[r] = (float)(2.0 * 3.14159265359 * wmu[r]);
+  }
+  void *dray;
+  TRY(scratch(27, hray.size(), &dray));
+  CUDA_TRY(cudaMemcpyAsync(dray, hray.data(), hray.size(), cudaMemcpyHostToDevice, g_ctx.stream));
+  const QuadConst *dqc = (const QuadConst *)dray;
+  const float *dw = (const float *)(dqc + nray);
+
+  // partial sums of the intensity reduction: blocks of 8 columns, at most 148 of them
+  // (a part without columns would add a zero)
+  const int kParts = (int)std::min<size_t>(148, (ncol + 7) / 8);
   void *dpart;
-  TRY(scratch(12, sizeof(double) * kParts * nf, &dpart));
+  TRY(scratch(12, sizeof(double) * kParts * nf * group, &dpart));
 
   // FP64 plain path buffers
   void *dwork = nullptr, *dmem = nullptr;
@@ -1486,32 +1547,33 @@ int lte_synthesis_impl(const m3d_atmos_t *atm, int nwin, int nf_win, const doubl
     TRY(scratch(11, sizeof(double) * plane * 3, &dmem));
   }
 
-  // a batch's opacity: every ray and window in one launch
-  if (nwin > 1) TRY(launch_opacity(in, vec, fp64, dchi, dS));
-  for (int r = 0; r < nray; r++) {
-    const double *v = vec + 3 * r;
-    if (nwin == 1) TRY(launch_opacity(in, v, fp64, dchi, dS));
-    // this ray's transfer units
-    const size_t ru = nwin > 1 ? plane * nz * (size_t)r : 0;
-    const void *rchi = (const char *)dchi + esz * ru, *rS = (const char *)dS + esz * ru;
+  for (int r0 = 0; r0 < nray; r0 += group) {
+    const int nr = std::min(group, nray - r0);
+    TRY(launch_opacity(in, vec + 3 * r0, d_vr + 3 * r0, nr, fp64, dchi, dS));
     if (!fp64) {
-      const QuadConst qc = quad_const(atm->ds_cm[2], v[2]);
+      float *top = (float *)dtop + plane * r0;
+      const RotCol *rot_r = (const RotCol *)drot + (size_t)r0 * nz;
       if (nf % 2 == 0) {
         // frequency pairs: 8-byte taps, the ray's rotation weights in shared memory
-        const size_t pairs = plane / 2;
-        LAUNCH_S(M3D_STAGE_SOLVE, k_quad_rot_column2, (int)((pairs + 255) / 256), 256, sizeof(RotCol) * nz, nf, nx, ny,
-                 nz, (const float *)rchi, (const float *)rS, (const RotCol *)drot + (size_t)r * nz, (const int *)dz0,
-                 atm->nslab, qc, pc, dtmax, Imax, (float *)dtop + plane * r);
+        const dim3 grid((unsigned)((plane / 2 + 255) / 256), nr);
+        LAUNCH_S(M3D_STAGE_SOLVE, k_quad_rot_column2, grid, 256, sizeof(RotCol) * nz, nf, nx, ny, nz,
+                 (const float *)dchi, (const float *)dS, rot_r, (const int *)dz0, atm->nslab, dqc + r0, pc, dtmax,
+                 Imax, top);
       } else {
-        LAUNCH_S(M3D_STAGE_SOLVE, k_quad_rot_column, (int)((plane + 255) / 256), 256, 0, nf, nx, ny, nz,
-                 (const float *)rchi, (const float *)rS, (const RotCol *)drot + (size_t)r * nz, (const int *)dz0,
-                 atm->nslab, qc, pc, dtmax, Imax, (float *)dtop + plane * r);
+        const dim3 grid((unsigned)((plane + 255) / 256), nr);
+        LAUNCH_S(M3D_STAGE_SOLVE, k_quad_rot_column, grid, 256, 0, nf, nx, ny, nz, (const float *)dchi,
+                 (const float *)dS, rot_r, (const int *)dz0, atm->nslab, dqc + r0, pc, dtmax, Imax, top);
       }
-      LAUNCH_S(M3D_STAGE_REDUCE, k_save_partial<float>, dim3((nf + 31) / 32, kParts), dim3(32, 8), 0, nf, (int)ncol,
-               dnu, (const float *)dtop + plane * r, (double *)dpart);
-      LAUNCH_S(M3D_STAGE_REDUCE, k_save_final, (nf + 127) / 128, 128, 0, nf, (int)ncol, kParts, (const double *)dpart,
-               die + (size_t)nf * r);
-    } else {
+      LAUNCH_S(M3D_STAGE_REDUCE, k_save_partial<float>, dim3((nf + 31) / 32, kParts, nr), dim3(32, 8), 0, nf,
+               (int)ncol, dnu, (const float *)top, (double *)dpart);
+      LAUNCH_S(M3D_STAGE_REDUCE, k_save_final, dim3((nf + 127) / 128, nr), 128, 0, nf, (int)ncol, kParts,
+               (const double *)dpart, die + (size_t)nf * r0);
+      continue;
+    }
+    for (int r = r0; r < r0 + nr; r++) {
+      const double *v = vec + 3 * r;
+      const double *rchi = (const double *)dchi + plane * nz * (size_t)(r - r0);
+      const double *rS = (const double *)dS + plane * nz * (size_t)(r - r0);
       for (int s = 0; s < atm->nslab; s++) {
         const int n = atm->slab_nz[s];
         m3d_slab_t sl;
@@ -1521,8 +1583,7 @@ int lte_synthesis_impl(const m3d_atmos_t *atm, int nwin, int nf_win, const doubl
         sl.maser_dtau_max = atm->maser_dtau_max;
         sl.maser_Inu_max = atm->maser_Inu_max;
         double *w = (double *)dwork;
-        LAUNCH(k_slab_in, grid_for(plane * n), 256, 0, plane, n, (const double *)rchi + plane * z0[s],
-               (const double *)rS + plane * z0[s], w, n);
+        LAUNCH(k_slab_in, grid_for(plane * n), 256, 0, plane, n, rchi + plane * z0[s], rS + plane * z0[s], w, n);
         LAUNCH(k_upstream_boundary<double>, grid_for(plane), 256, 0, nf, nx, ny, n, 1, w, s == 0 ? M3D_BND_PCHIP : M3D_BND_MEM,
                (const double *)dmem, pc, (const float *)nullptr, (const float *)nullptr, (const double *)nullptr);
         const float bottom = (float)((double)z0[s] * atm->ds_code[2]);
@@ -1536,32 +1597,16 @@ int lte_synthesis_impl(const m3d_atmos_t *atm, int nwin, int nf_win, const doubl
       }
       CUDA_TRY(cudaMemcpyAsync((double *)dtop + plane * r, (double *)dmem + 2 * plane, sizeof(double) * plane,
                                cudaMemcpyDeviceToDevice, g_ctx.stream));
-      LAUNCH_S(M3D_STAGE_REDUCE, k_save_partial<double>, dim3((nf + 31) / 32, kParts), dim3(32, 8), 0, nf,
-               (int)ncol, dnu, (const double *)dtop + plane * r, (double *)dpart);
-      LAUNCH_S(M3D_STAGE_REDUCE, k_save_final, (nf + 127) / 128, 128, 0, nf, (int)ncol, kParts, (const double *)dpart,
-               die + (size_t)nf * r);
     }
+    LAUNCH_S(M3D_STAGE_REDUCE, k_save_partial<double>, dim3((nf + 31) / 32, kParts, nr), dim3(32, 8), 0, nf,
+             (int)ncol, dnu, (const double *)dtop + plane * r0, (double *)dpart);
+    LAUNCH_S(M3D_STAGE_REDUCE, k_save_final, dim3((nf + 127) / 128, nr), 128, 0, nf, (int)ncol, kParts,
+             (const double *)dpart, die + (size_t)nf * r0);
   }
+  LAUNCH_S(M3D_STAGE_REDUCE, k_flux, (nf + 127) / 128, 128, 0, nf, nray, dw, (const float *)die, dflux);
   TRY(st.finish());
-  // flux = 2 pi sum_mu wmu ie (rt_patch_mod.f90:4193-4200), ie now on the host or device
-  std::vector<float> hie((size_t)nf * nray);
-  if (st.device()) {
-    CUDA_TRY(cudaMemcpyAsync(hie.data(), ie, sizeof(float) * hie.size(), cudaMemcpyDeviceToHost, g_ctx.stream));
-    CUDA_TRY(cudaStreamSynchronize(g_ctx.stream));
-  } else {
-    memcpy(hie.data(), ie, sizeof(float) * hie.size());
-  }
-  std::vector<float> hflux(nf, 0.0f);
-  for (int r = 0; r < nray; r++) {
-    const float w = (float)(2.0 * 3.14159265359 * wmu[r]);
-    for (int f = 0; f < nf; f++) hflux[f] = fmaf(w, hie[(size_t)f + (size_t)nf * r], hflux[f]);
-  }
-  if (st.device()) {
-    CUDA_TRY(cudaMemcpyAsync(flux, hflux.data(), sizeof(float) * nf, cudaMemcpyHostToDevice, g_ctx.stream));
-    CUDA_TRY(cudaStreamSynchronize(g_ctx.stream));
-  } else {
-    memcpy(flux, hflux.data(), sizeof(float) * nf);
-  }
+  // the caller's results are complete on return, whichever stream reads them
+  if (st.device()) CUDA_TRY(cudaStreamSynchronize(g_ctx.stream));
   return M3D_OK;
 }
 

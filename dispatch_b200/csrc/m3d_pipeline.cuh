@@ -79,10 +79,11 @@ __device__ __forceinline__ float point_xhat(float chi_c, float h_kT, double nu) 
   return chi_c + chi_c * Bnu;
 }
 
+// One warp per cell, for the windows and line lists that the lane kernel below does not
+// take: fewer than 8 frequencies, or reach_in with other than 32.
 // Shared memory: the two QLG tables, then per warp xhat, logref, chi_l, eta_l (nf each)
-template <typename TO>
 __global__ void __launch_bounds__(256) k_lte_opacity_units(AtmosDev A, GridArgs G, const double *nu, double v0,
-                                                           double v1, double v2, TO *chi_out, TO *S_out,
+                                                           double v1, double v2, float *chi_out, float *S_out,
                                                            const float2 *tab) {
   extern __shared__ float smem[];
   float2 *s_tab = reinterpret_cast<float2 *>(smem);
@@ -116,12 +117,8 @@ __global__ void __launch_bounds__(256) k_lte_opacity_units(AtmosDev A, GridArgs 
     }
     __syncwarp();
     for (int f = lane; f < nf; f += 32) {
-      TO co, so;
-      if constexpr (sizeof(TO) == 4) {
-        point_units(chi_c, h_kT, nu[f], s_chi[f], s_eta[f], A.maser_chi_floor, co, so);
-      } else {
-        point_units((double)chi_c, (double)T, nu[f], (double)s_chi[f], (double)s_eta[f], (double)A.maser_chi_floor, co, so);
-      }
+      float co, so;
+      point_units(chi_c, h_kT, nu[f], s_chi[f], s_eta[f], A.maser_chi_floor, co, so);
       chi_out[(size_t)f + (size_t)nf * cell] = co;
       S_out[(size_t)f + (size_t)nf * cell] = so;
     }
@@ -141,51 +138,42 @@ __global__ void __launch_bounds__(256) k_lte_opacity_units(AtmosDev A, GridArgs 
 // the spot otherwise; the accumulated line opacity there is picked out of the
 // register array.  Results are bit-identical to k_lte_opacity_units.
 // ---------------------------------------------------------------------------
+// The window of a line as a lane's NF registers hold it.  The first NF/2 hold the
+// lane's frequencies o, o+1, .., the last NF/2 its last NF/2 ones, so both ends of the
+// lane's nl <= NF frequencies (nl >= NF/2) sit at fixed registers, whatever nl is; the
+// NF - nl frequencies that both halves hold are evaluated twice, to the same bits.
+// Register k stands for the abscissa offset (float)k + klo or khi (an exact integer
+// sum) and lies inside the line's window where alo <= k+1 <= blo, or ahi .. bhi.
+struct LaneWin { float klo, khi; int alo, blo, ahi, bhi; };
+
 // One line's profile over the window into chl.  far: every window point lies
 // beyond the QLG table, where G and W are the last node's at every point and the
-// evaluation is qlg_eval's with them folded in; full: the line covers the whole
-// window, which then runs without per-point predicates (with fa = 1 the offset
-// (float)f + kfa is (float)f).  MK: every point's 1 + xs^2 is below 2^126, so the
-// reciprocal is rcp_markstein's.  All forms give the bits of the general one.
-template <int NF, bool MK>
+// evaluation is qlg_eval's with them folded in; full: the line covers the lane's whole
+// window, which then runs without per-point predicates; OFF: the lane's registers do
+// not start at the window's first frequency or hold it unevenly, so the offsets are
+// added even where the line covers the window.  MK: every point's 1 + xs^2 is below
+// 2^126, so the reciprocal is rcp_markstein's.  All forms give the bits of the general
+// one.
+template <int NF, bool MK, bool OFF>
 __device__ __forceinline__ void deposit_window(float (&chl)[NF], const float2 *s_tab, const QlgCoef &cf, float x0,
-                                               float kfa, int fa, int fb, bool full, bool far) {
-  if (far) {
-    const float2 gw = s_tab[QLG_NTAB - 1];
-    const float p1 = fmaf(cf.cZH, gw.y, cf.cL2);
-    const float gg = gw.x * cf.gG;
-    if (full) {
+                                               const LaneWin &w, bool full, bool far) {
+  const float2 gw = s_tab[QLG_NTAB - 1];
+  const float p1 = fmaf(cf.cZH, gw.y, cf.cL2);
+  const float gg = gw.x * cf.gG;
 #pragma unroll
-      for (int f = 0; f < NF; f++) {
-        const float xs = fabsf(x0 + (float)f) * cf.ih;
+  for (int f = 0; f < NF; f++) {
+    const bool hi = f >= NF / 2;
+    if (full || (f + 1 >= (hi ? w.ahi : w.alo) && f + 1 <= (hi ? w.bhi : w.blo))) {
+      const float x = x0 + ((float)f + (hi ? w.khi : w.klo));
+      float K;
+      if (far) {
+        const float xs = fabsf(x) * cf.ih;
         const float L = qlg_rcp<MK>(1.0f + xs * xs);
-        const float K = fmaf(L, fmaf(L, p1, cf.bL), gg);
-        chl[f] = fmaf(K, 1.0f, chl[f]);
+        K = fmaf(L, fmaf(L, p1, cf.bL), gg);
+      } else {
+        K = qlg_eval<MK>(s_tab, cf, x);
       }
-    } else {
-#pragma unroll
-      for (int f = 0; f < NF; f++) {
-        if (f + 1 >= fa && f + 1 <= fb) {
-          const float xs = fabsf(x0 + ((float)f + kfa)) * cf.ih;
-          const float L = qlg_rcp<MK>(1.0f + xs * xs);
-          const float K = fmaf(L, fmaf(L, p1, cf.bL), gg);
-          chl[f] = fmaf(K, 1.0f, chl[f]);
-        }
-      }
-    }
-  } else if (full) {
-#pragma unroll
-    for (int f = 0; f < NF; f++) {
-      const float K = qlg_eval<MK>(s_tab, cf, x0 + (float)f);
       chl[f] = fmaf(K, 1.0f, chl[f]);
-    }
-  } else {
-#pragma unroll
-    for (int f = 0; f < NF; f++) {
-      if (f + 1 >= fa && f + 1 <= fb) {
-        const float K = qlg_eval<MK>(s_tab, cf, x0 + ((float)f + kfa));
-        chl[f] = fmaf(K, 1.0f, chl[f]);
-      }
     }
   }
 }
@@ -219,12 +207,12 @@ __device__ __forceinline__ float2 lds_node(unsigned addr) {
   return v;
 }
 
-template <int NF, bool FULL, bool FAR>
+template <int NF, bool FULL, bool FAR, bool OFF>
 __device__ __forceinline__ void deposit_window_x2(float (&chl)[NF], const float2 *s_tab, const QlgCoef &cf,
-                                                  float x0, float kfa, int fa, int fb) {
-  static_assert(NF % 2 == 0, "pairs of window points");
+                                                  float x0, const LaneWin &w) {
+  static_assert(NF % 4 == 0, "pairs of window points, in two halves");
   const f32x2 X0 = splat2(x0), IH = splat2(cf.ih), ONE = splat2(1.0f), BL = splat2(cf.bL);
-  const f32x2 KF = splat2(kfa);
+  const f32x2 KLO = splat2(w.klo), KHI = splat2(w.khi);
   f32x2 P1 = 0, GG = 0, CZH = 0, CL2 = 0, GGc = 0;
   unsigned base = 0;
   if (FAR) {
@@ -241,7 +229,7 @@ __device__ __forceinline__ void deposit_window_x2(float (&chl)[NF], const float2
 #pragma unroll
   for (int k = 0; k < NF / 2; k++) {
     f32x2 F = pk2((float)(2 * k), (float)(2 * k + 1));
-    if (!FULL) F = add2(F, KF);  // (float)f + kfa, exact
+    if (!FULL || OFF) F = add2(F, 2 * k >= NF / 2 ? KHI : KLO);  // exact
     const f32x2 x = add2(X0, F);
     const f32x2 xs = mul2(x, IH);
     float xa, xb;
@@ -271,8 +259,9 @@ __device__ __forceinline__ void deposit_window_x2(float (&chl)[NF], const float2
     if (!FULL) {
       float ka, kb;
       up2(K, ka, kb);
-      ka = (2 * k + 1 >= fa && 2 * k + 1 <= fb) ? ka : 0.0f;
-      kb = (2 * k + 2 >= fa && 2 * k + 2 <= fb) ? kb : 0.0f;
+      const int a = 2 * k >= NF / 2 ? w.ahi : w.alo, b = 2 * k >= NF / 2 ? w.bhi : w.blo;
+      ka = (2 * k + 1 >= a && 2 * k + 1 <= b) ? ka : 0.0f;
+      kb = (2 * k + 2 >= a && 2 * k + 2 <= b) ? kb : 0.0f;
       K = pk2(ka, kb);
     }
     float lo, hi;
@@ -282,15 +271,15 @@ __device__ __forceinline__ void deposit_window_x2(float (&chl)[NF], const float2
   }
 }
 
-template <int NF>
+template <int NF, bool OFF>
 __device__ __forceinline__ void deposit_window_mk(float (&chl)[NF], const float2 *s_tab, const QlgCoef &cf, float x0,
-                                                  float kfa, int fa, int fb, bool full, bool far) {
+                                                  const LaneWin &w, bool full, bool far) {
   if (far) {
-    if (full) deposit_window_x2<NF, true, true>(chl, s_tab, cf, x0, kfa, fa, fb);
-    else deposit_window_x2<NF, false, true>(chl, s_tab, cf, x0, kfa, fa, fb);
+    if (full) deposit_window_x2<NF, true, true, OFF>(chl, s_tab, cf, x0, w);
+    else deposit_window_x2<NF, false, true, OFF>(chl, s_tab, cf, x0, w);
   } else {
-    if (full) deposit_window_x2<NF, true, false>(chl, s_tab, cf, x0, kfa, fa, fb);
-    else deposit_window_x2<NF, false, false>(chl, s_tab, cf, x0, kfa, fa, fb);
+    if (full) deposit_window_x2<NF, true, false, OFF>(chl, s_tab, cf, x0, w);
+    else deposit_window_x2<NF, false, false, OFF>(chl, s_tab, cf, x0, w);
   }
 }
 
@@ -313,43 +302,70 @@ __device__ __forceinline__ float pick(const float (&a)[NF], int i) {
   return v;
 }
 
+// Threads of the lane kernel's block, one block per SM: as many warps as the NF
+// registers of chi_l and the line's working set leave room for (64, 80, 96 and 128
+// registers a thread)
+__host__ __device__ constexpr int lane_threads(int NF) { return NF <= 16 ? 1024 : NF <= 32 ? 768 : NF <= 48 ? 640 : 512; }
+
 // REACH: the line list carries reach_in (has_reach): the lines select_lines kept,
 // and lines centred beyond the window take the unfloored reference at the nearer
 // end, no peak test and a window capped by their reach (linelist_mod.f90:844-854, 914-921)
 // CHIL: write the line opacity chi_l of the window itself to chi_out (S_out unused):
 // the input of the adjoint's transfer units
-// BATCH: nray directions (vr, 3 each) and nwin windows of NF frequencies in one
-// launch, each window with its own grid Gw[w] and frequencies nu + w NF; the warps run
-// over (ray, window, cell) with the cells of a window padded to whole warps, so a warp
-// holds one ray and window, and a cell's row of every window goes to chi_out +
-// ray ncell nwin NF + nwin NF cell + w NF: per ray the rows of one window of nwin NF
-// frequencies, which the column solvers take as they are
-template <int NF, typename TO, bool REACH, bool CHIL = false, bool BATCH = false>
-__global__ void __launch_bounds__(768, 1) k_lte_opacity_units_lane(AtmosDev A, GridArgs G0, const double *nu0,
-                                                                   double v0_, double v1_, double v2_, TO *chi_out,
-                                                                   TO *S_out, const float2 *tab, const GridArgs *Gw,
-                                                                   int nwin, const double *vr, int nray) {
+// WINS: nwin windows of NF frequencies, each with its own grid Gw[w] and frequencies
+// nu + w NF
+// PAD: a window of nf <= NF frequencies (nf >= NF/2); MULTI: a window of nf > NF, a cell
+// taking P lanes (a power of two) that hold a P-th of the window each; the lanes of a
+// cell repeat its line's set-up and exchange the line opacity at the line's node.
+//
+// nray directions (vr, 3 each) share the launch: the (ray, cell) pairs of a window run
+// in one sequence over the warps, so a small atmosphere's rays fill the GPU together
+// (24^3 cells are 432 warps a ray; 13 rays a launch each took 12.6 ms) and a column's
+// last warp takes the next ray's cells.  Per ray the rows go to chi_out + ray ncell
+// nwin nf, where the column solvers take them as those of one window of nwin nf
+// frequencies.  One block stays on each SM; its warps start on units that alternate
+// over the blocks, so that few of them spread evenly over the SMs, and fetch their next
+// from a counter (*next, zero at the launch): a unit's time follows its cells' lines,
+// and warps that strode over a fixed share of the units left the 96^3 cube 4 % slower
+// than blocks handed out by the hardware.
+template <int NF, bool REACH, bool CHIL = false, bool WINS = false, bool PAD = false, bool MULTI = false>
+__global__ void __launch_bounds__(lane_threads(NF), 1)
+    k_lte_opacity_units_lane(AtmosDev A, GridArgs G0, const double *nu0, float *chi_out, float *S_out,
+                             const float2 *tab, const GridArgs *Gw, int nwin, const double *vr, int nray, int P_,
+                             int *next) {
   extern __shared__ float smem[];
   float2 *s_tab = reinterpret_cast<float2 *>(smem);
   stage_tables(s_tab, tab);
+  constexpr bool OFF = PAD || MULTI;
+  static_assert(!(WINS && OFF), "window batches of a fixed window size");
   const float ex_cutoff = -85.0f, voigt_peak = 0.5641895835f, sqrt_pi = 1.7724538509f;
   const float lt = logf_m3d(G0.tol / voigt_peak);
   const int ncell = A.ncell;
-  const int nthreads = gridDim.x * blockDim.x;
-  const int ncell_pad = (ncell + 31) / 32 * 32;
-  const int nvc = BATCH ? ncell_pad * nwin * nray : ncell_pad;
-  for (int vc = blockIdx.x * blockDim.x + threadIdx.x; vc < nvc; vc += nthreads) {
-    const int ray = BATCH ? vc / (ncell_pad * nwin) : 0;
-    const int wc = BATCH ? vc - ray * (ncell_pad * nwin) : vc;
-    const int w = BATCH ? wc / ncell_pad : 0;
-    const int cell = BATCH ? wc - w * ncell_pad : wc;
-    const GridArgs G = BATCH ? Gw[w] : G0;
-    const double *nu = BATCH ? nu0 + (size_t)NF * w : nu0;
-    const double v0 = BATCH ? vr[3 * ray] : v0_, v1 = BATCH ? vr[3 * ray + 1] : v1_, v2 = BATCH ? vr[3 * ray + 2] : v2_;
-    const size_t row = BATCH ? (size_t)ray * ncell * nwin * NF + (size_t)NF * nwin * cell + (size_t)NF * w
-                             : (size_t)NF * cell;
-    const bool live = cell < ncell;
-    const int cs = live ? cell : ncell - 1;
+  const int nf = OFF ? G0.nf : NF;
+  const int P = MULTI ? P_ : 1;
+  const int lane = threadIdx.x & 31;
+  // this lane's frequencies o .. o + nl of the window
+  const int sub = lane & (P - 1);
+  const int o = MULTI ? (sub * nf) / P : 0;
+  const int nl = MULTI ? ((sub + 1) * nf) / P - o : nf;
+  const int pad = NF - nl;
+  const unsigned cellmask = MULTI ? (P == 32 ? 0xffffffffu : ((1u << P) - 1u) << (lane & ~(P - 1))) : 0u;
+  const int cw = 32 / P;                                      // cells per warp
+  const int upw = (int)(((long long)nray * ncell + cw - 1) / cw);   // warps' units per window
+  const int nunit = WINS ? upw * nwin : upw;
+  auto fetch = [&]() {
+    int v = 0;
+    if ((threadIdx.x & 31) == 0) v = atomicAdd(next, 1) + gridDim.x * (blockDim.x >> 5);
+    return __shfl_sync(0xffffffffu, v, 0);
+  };
+  for (int u = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; u < nunit; u = fetch()) {
+    const int w = WINS ? u / upw : 0;
+    const long long rc = min((long long)(u - w * upw) * cw + lane / P, (long long)nray * ncell - 1);
+    const int ray = (int)(rc / ncell);
+    const int cs = (int)(rc - (long long)ray * ncell);
+    const GridArgs G = WINS ? Gw[w] : G0;
+    const double *nu = WINS ? nu0 + (size_t)NF * w : nu0;
+    const double v0 = vr[3 * ray], v1 = vr[3 * ray + 1], v2 = vr[3 * ray + 2];
     const float T = A.temp[cs], chi_c = A.chi_c[cs];
     const float h_kT = (float)(M3D_H_K / (double)T);
     float chl[NF];
@@ -358,10 +374,10 @@ __global__ void __launch_bounds__(768, 1) k_lte_opacity_units_lane(AtmosDev A, G
     const float vproj = (float)((v0 * (double)A.vx[cs] + v1 * (double)A.vy[cs]) + v2 * (double)A.vz[cs]);
     const float ekt = A.e_kT[cs], ne = A.ne[cs], tothi = A.tothi[cs], starkpe = A.stark_pe[cs];
     // xhat and logref at the window edges
-    const float x_lo = point_xhat(chi_c, h_kT, nu[0]), x_hi = point_xhat(chi_c, h_kT, nu[NF - 1]);
+    const float x_lo = point_xhat(chi_c, h_kT, nu[0]), x_hi = point_xhat(chi_c, h_kT, nu[nf - 1]);
     const float lr_lo = x_lo > 0.0f ? lt + logf_m3d(x_lo) : -FLT_MAX;
     const float lr_hi = x_hi > 0.0f ? lt + logf_m3d(x_hi) : -FLT_MAX;
-    const double llam_hi = G.llam[NF - 1];
+    const double llam_hi = G.llam[nf - 1];
     for (int sp = 0; sp < A.nspecies; sp++) {
       const SpeciesDev &Sd = A.species[sp];
       const LineArgs &L = Sd.L;
@@ -379,18 +395,21 @@ __global__ void __launch_bounds__(768, 1) k_lte_opacity_units_lane(AtmosDev A, G
         const double llc = L.llam0[l] - (double)vproj;
         const double pos = (llc - G.llam1) * G.inv_dllam;
         const int ic = lround_d(pos) + 1;
-        const int f0 = ic < 1 ? 1 : (ic > NF ? NF : ic);
+        const int f0 = ic < 1 ? 1 : (ic > nf ? nf : ic);
         // the nearest node's xhat, its log and the line opacity there: a line centred
         // outside the window -- nearly all of them -- lands on an edge, whose values
         // are at hand; an interior node forms them (one branch, taken rarely)
         float cont0, lr0, chl0;
         if (f0 == 1) { cont0 = x_lo; lr0 = lr_lo; chl0 = chl[0]; }
-        else if (f0 == NF) { cont0 = x_hi; lr0 = lr_hi; chl0 = chl[NF - 1]; }
+        else if (f0 == nf) { cont0 = x_hi; lr0 = lr_hi; chl0 = chl[NF - 1]; }
         else {
           cont0 = point_xhat(chi_c, h_kT, nu[f0 - 1]);
           lr0 = cont0 > 0.0f ? lt + logf_m3d(cont0) : -FLT_MAX;
-          chl0 = pick<NF>(chl, f0 - 1);
+          const int i = f0 - 1 - o;
+          chl0 = pick<NF>(chl, OFF && i >= NF / 2 ? i + pad : i);
         }
+        // the lane that holds the node: the largest with o <= f0 - 1
+        if (MULTI) chl0 = __shfl_sync(cellmask, chl0, (f0 * P - 1) / nf, P);
         float refl = G.tol * cont0;
         float lref, cap = FLT_MAX;
         const bool outside = REACH && (llc < G.llam[0] || llc > llam_hi);
@@ -411,71 +430,87 @@ __global__ void __launch_bounds__(768, 1) k_lte_opacity_units_lane(AtmosDev A, G
         // (llam(f0) - llc)/dllam; at f0 = 1 it is -pos exactly (the rounded difference
         // and product are odd in their sign)
         const float x1 = f0 == 1 ? (float)(-pos)
-                                 : (float)(((f0 == NF ? llam_hi : G.llam[f0 - 1]) - llc) * G.inv_dllam);
+                                 : (float)(((f0 == nf ? llam_hi : G.llam[f0 - 1]) - llc) * G.inv_dllam);
         const QlgCoef cf = qlg_setup(a, qw.D, qw.SQ, S);
         const float hw = qlg_halfwidth(qw, a, S, refl, arg - lref);
-        const int noff = lround_pos(fminf(fminf(hw, cap), (float)(NF + abs(ic))));
+        const int noff = lround_pos(fminf(fminf(hw, cap), (float)(nf + abs(ic))));
         const int fa = ic - noff > 1 ? ic - noff : 1;
-        const int fb = ic + noff < NF ? ic + noff : NF;
-        if (fa > fb) continue;
+        const int fb = ic + noff < nf ? ic + noff : nf;
+        // the part of the line's window that this lane holds
+        const int ga = MULTI ? max(fa, o + 1) : fa, gb = MULTI ? min(fb, o + nl) : fb;
+        if (ga > gb) continue;
         const float x0 = x1 - (float)(f0 - fa);
-        const float kfa = (float)(1 - fa);    // (float)(f + 1 - fa) = (float)f + kfa, exactly
+        LaneWin lw;
+        lw.klo = (float)(o + 1 - fa);         // (float)(f + 1 - fa) = (float)k + klo, exactly
+        lw.khi = OFF ? (float)(o - pad + 1 - fa) : lw.klo;
+        lw.alo = OFF ? fa - o : fa;
+        lw.blo = OFF ? fb - o : fb;
+        lw.ahi = OFF ? lw.alo + pad : fa;
+        lw.bhi = OFF ? lw.blo + pad : fb;
         // Far wing: when even the window point nearest the line centre snaps to the
         // last table node, G and W are the same two constants at every point, and the
         // evaluation is qlg_eval's with them folded in.  The snapped index is monotone
         // in |x| (rounded products are monotone), so the nearer window end decides.
-        const float xe = x0 + (float)(fb - fa);
-        const float xnear = (x0 > 0.0f) ? x0 : ((xe < 0.0f) ? -xe : 0.0f);
+        const float xb = MULTI ? x0 + (float)(ga - fa) : x0;
+        const float xe = x0 + (float)(gb - fa);
+        const float xnear = (xb > 0.0f) ? xb : ((xe < 0.0f) ? -xe : 0.0f);
         // A window over the whole frequency range -- most lines -- runs without
-        // per-point predicates, and with fa = 1 the offset (float)f + kfa is (float)f.
+        // per-point predicates, and with fa = 1 the offset (float)f + klo is (float)f.
         // The far-wing and whole-window forms are taken only when every converged
         // lane of the warp qualifies: the general forms give the same values where
         // the special ones apply, so the warp never runs two forms of one line.
         const unsigned conv = __activemask();
-        const bool full = __all_sync(conv, fa == 1 && fb == NF);
+        const bool full = __all_sync(conv, fa <= o + 1 && fb >= o + nl);
         const bool far = __all_sync(conv, fminf((xnear * cf.ih) * 800.0f, 9019.0f) >= 9018.5f);
         // The window's largest |x| ih bounds every point's 1 + xs^2 (rounded products
         // are monotone): at most 2^62 keeps it under 2^126, where rcp_markstein is
         // exact.  One vote per line picks the reciprocal for the whole window.
-        const float xmax = fmaxf(fabsf(x0), fabsf(xe)) * cf.ih;
+        const float xmax = fmaxf(fabsf(xb), fabsf(xe)) * cf.ih;
         if (__all_sync(conv, xmax <= 4611686018427387904.0f))
-          deposit_window_mk<NF>(chl, s_tab, cf, x0, kfa, fa, fb, full, far);
+          deposit_window_mk<NF, OFF>(chl, s_tab, cf, x0, lw, full, far);
         else
-          deposit_window<NF, false>(chl, s_tab, cf, x0, kfa, fa, fb, full, far);
+          deposit_window<NF, false, OFF>(chl, s_tab, cf, x0, lw, full, far);
       }
     }
+    // this lane's row, its place formed again rather than held through the line loop
+    size_t row;
+    {
+      int ue = u;
+      asm volatile("" : "+r"(ue));
+      const int we = WINS ? ue / upw : 0;
+      const long long re = (long long)(ue - we * upw) * cw + (threadIdx.x & 31) / P;
+      if (re >= (long long)nray * ncell) continue;
+      row = WINS ? (size_t)NF * nwin * (size_t)re + (size_t)NF * we : (size_t)nf * (size_t)re;
+    }
+    float *co = chi_out + row, *so = S_out + row;
     if (CHIL) {
-      if (live) {
-        float *co = reinterpret_cast<float *>(chi_out) + row;
 #pragma unroll
-        for (int f = 0; f < NF; f += 4)
-          *reinterpret_cast<float4 *>(co + f) = make_float4(chl[f], chl[f + 1], chl[f + 2], chl[f + 3]);
-      }
+      for (int f = 0; f < NF; f += 4)
+        *reinterpret_cast<float4 *>(co + f) = make_float4(chl[f], chl[f + 1], chl[f + 2], chl[f + 3]);
       continue;
     }
-    // epilogue: transfer units, written as 16-byte stores of this cell's row
-    if (live) {
-      TO *co = chi_out + row, *so = S_out + row;
+    // epilogue: transfer units, written as 16-byte stores of this cell's row where the
+    // row is a whole number of them
+    if (!OFF) {
 #pragma unroll
       for (int f = 0; f < NF; f += 4) {
-        TO c4[4], s4[4];
+        float c4[4], s4[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-          if constexpr (sizeof(TO) == 4) {
-            point_units(chi_c, h_kT, nu[f + k], chl[f + k], chl[f + k], A.maser_chi_floor, c4[k], s4[k]);
-          } else {
-            point_units((double)chi_c, (double)T, nu[f + k], (double)chl[f + k], (double)chl[f + k],
-                        (double)A.maser_chi_floor, c4[k], s4[k]);
-          }
-        }
-        if constexpr (sizeof(TO) == 4) {
-          *reinterpret_cast<float4 *>(co + f) = make_float4(c4[0], c4[1], c4[2], c4[3]);
-          *reinterpret_cast<float4 *>(so + f) = make_float4(s4[0], s4[1], s4[2], s4[3]);
-        } else {
-          reinterpret_cast<double2 *>(co + f)[0] = make_double2(c4[0], c4[1]);
-          reinterpret_cast<double2 *>(co + f)[1] = make_double2(c4[2], c4[3]);
-          reinterpret_cast<double2 *>(so + f)[0] = make_double2(s4[0], s4[1]);
-          reinterpret_cast<double2 *>(so + f)[1] = make_double2(s4[2], s4[3]);
+        for (int k = 0; k < 4; k++)
+          point_units(chi_c, h_kT, nu[f + k], chl[f + k], chl[f + k], A.maser_chi_floor, c4[k], s4[k]);
+        *reinterpret_cast<float4 *>(co + f) = make_float4(c4[0], c4[1], c4[2], c4[3]);
+        *reinterpret_cast<float4 *>(so + f) = make_float4(s4[0], s4[1], s4[2], s4[3]);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < NF; k++) {
+        // the frequencies both halves hold are written once, from the first
+        if (k < NF / 2 || k - pad >= NF / 2) {
+          const int f = o + (k < NF / 2 ? k : k - pad);
+          float c1, s1;
+          point_units(chi_c, h_kT, nu[f], chl[k], chl[k], A.maser_chi_floor, c1, s1);
+          co[f] = c1;
+          so[f] = s1;
         }
       }
     }
@@ -554,32 +589,34 @@ struct ChlF64<0> {
   __device__ __forceinline__ double &operator[](int i) { return p[i]; }
 };
 
-// BATCH: nray directions and nwin windows in one launch, as
-// k_lte_opacity_units_lane<..., BATCH> (NF > 0)
-template <int NF, bool BATCH = false>
+// nray directions share the launch, and with WINS nwin windows (NF > 0), as in
+// k_lte_opacity_units_lane
+template <int NF, bool WINS = false>
 __global__ void __launch_bounds__(256) k_lte_opacity_units_f64(AtmosDev A, GridArgs G0, const double *nu0,
-                                                               double v0_, double v1_, double v2_, double *chi_out,
-                                                               double *S_out, const double2 *tab, const GridArgs *Gw,
-                                                               int nwin, const double *vr, int nray) {
-  static_assert(!BATCH || NF > 0, "window batches of a fixed window size");
+                                                               double *chi_out, double *S_out, const double2 *tab,
+                                                               const GridArgs *Gw, int nwin, const double *vr,
+                                                               int nray) {
+  static_assert(!WINS || NF > 0, "window batches of a fixed window size");
   const double ex_cutoff = -85.0, voigt_peak = 0.56418958354775628, sqrt_pi = 1.7724538509055160;
   const double tol = (double)G0.tol, flo_scale = (double)G0.flo_scale;
   const double lt = log(tol / voigt_peak);
   const int ncell = A.ncell;
   const int nf = NF > 0 ? NF : G0.nf;
-  const int nvc = BATCH ? ncell * nwin * nray : ncell;
-  for (int vc = blockIdx.x * blockDim.x + threadIdx.x; vc < nvc; vc += gridDim.x * blockDim.x) {
-    const int ray = BATCH ? vc / (ncell * nwin) : 0;
-    const int wc = BATCH ? vc - ray * (ncell * nwin) : vc;
-    const int w = BATCH ? wc / ncell : 0;
-    const int cell = BATCH ? wc - w * ncell : wc;
-    const GridArgs G = BATCH ? Gw[w] : G0;
-    const double *nu = BATCH ? nu0 + (size_t)nf * w : nu0;
-    const double v0 = BATCH ? vr[3 * ray] : v0_, v1 = BATCH ? vr[3 * ray + 1] : v1_, v2 = BATCH ? vr[3 * ray + 2] : v2_;
+  const long long nrc = (long long)nray * ncell;
+  const long long nvc = WINS ? nrc * nwin : nrc;
+  for (long long vc = blockIdx.x * (long long)blockDim.x + threadIdx.x; vc < nvc;
+       vc += (long long)gridDim.x * blockDim.x) {
+    const int w = WINS ? (int)(vc / nrc) : 0;
+    const long long rc = vc - w * nrc;
+    const int ray = (int)(rc / ncell);
+    const int cell = (int)(rc - (long long)ray * ncell);
+    const GridArgs G = WINS ? Gw[w] : G0;
+    const double *nu = WINS ? nu0 + (size_t)nf * w : nu0;
+    const double v0 = vr[3 * ray], v1 = vr[3 * ray + 1], v2 = vr[3 * ray + 2];
     const double sdl = G.inv_dllam;
     const double T = A.temp[cell], chi_c = A.chi_c[cell];
-    const size_t row = BATCH ? (size_t)ray * ncell * nwin * nf + (size_t)nf * nwin * cell + (size_t)nf * w
-                             : (size_t)nf * cell;
+    const size_t row = WINS ? (size_t)ray * ncell * nwin * nf + (size_t)nf * nwin * cell + (size_t)nf * w
+                            : (size_t)nf * (size_t)rc;
     double *co = chi_out + row, *so = S_out + row;
     ChlF64<NF> chl(co);
 #pragma unroll
@@ -710,15 +747,21 @@ __device__ __forceinline__ void combine(const Taps &t, const RotCol &r, float &x
   sv = fmaf(r.d, t.s22, w);
 }
 
-// chi, S: (nf, nx, ny, nz) unrotated transfer units of the whole column; rot: per
-// global plane; slab_z0: first global plane of each slab (nslab + 1 entries).
+// chi, S: (nf, nx, ny, nz) unrotated transfer units of the whole column, one ray after
+// the other along grid.y; rot: per global plane, qcs: per ray; slab_z0: first global
+// plane of each slab (nslab + 1 entries).
 __global__ void __launch_bounds__(256) k_quad_rot_column(int nf, int nx, int ny, int nz, const float *chi,
                                                          const float *S, const RotCol *rot, const int *slab_z0,
-                                                         int nslab, QuadConst qc, PchipConst pc, float dtmax,
+                                                         int nslab, const QuadConst *qcs, PchipConst pc, float dtmax,
                                                          float Imax, float *I_top) {
   const size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const size_t plane = (size_t)nf * nx * ny;
   if (g >= plane) return;
+  const QuadConst qc = qcs[blockIdx.y];
+  chi += plane * nz * blockIdx.y;
+  S += plane * nz * blockIdx.y;
+  rot += (size_t)nz * blockIdx.y;
+  I_top += plane * blockIdx.y;
   const int f = (int)(g % nf), x = (int)((g / nf) % nx), y = (int)(g / ((size_t)nf * nx));
   // PCHIP ghost below the bottom slab from its unrotated planes 1 and 2
   float gx, gs, gI;
@@ -813,9 +856,11 @@ __device__ __forceinline__ float pchip_ghost(float y1, float y2, const PchipCons
 // per SM (79 registers, no spills) measured 11 % faster than the unbounded 97.
 __global__ void __launch_bounds__(256, 3) k_quad_rot_column2(int nf, int nx, int ny, int nz, const float *chi,
                                                           const float *S, const RotCol *rot, const int *slab_z0,
-                                                          int nslab, QuadConst qc, PchipConst pc, float dtmax,
-                                                          float Imax, float *I_top) {
+                                                          int nslab, const QuadConst *qcs, PchipConst pc,
+                                                          float dtmax, float Imax, float *I_top) {
   extern __shared__ RotCol s_rot[];
+  const QuadConst qc = qcs[blockIdx.y];
+  rot += (size_t)nz * blockIdx.y;
   for (int i = threadIdx.x; i < nz; i += blockDim.x) s_rot[i] = rot[i];
   __syncthreads();
   const int nf2 = nf >> 1;
@@ -823,7 +868,8 @@ __global__ void __launch_bounds__(256, 3) k_quad_rot_column2(int nf, int nx, int
   const size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (g >= plane) return;
   const int f2 = (int)(g % nf2), x = (int)((g / nf2) % nx), y = (int)(g / ((size_t)nf2 * nx));
-  const float2 *chi2 = reinterpret_cast<const float2 *>(chi), *S2 = reinterpret_cast<const float2 *>(S);
+  const float2 *chi2 = reinterpret_cast<const float2 *>(chi) + plane * nz * blockIdx.y;
+  const float2 *S2 = reinterpret_cast<const float2 *>(S) + plane * nz * blockIdx.y;
   const float rdsup = qc.rdsup, dsup1 = qc.dsup1, dsup2 = qc.dsup2;
   // PCHIP ghost below the bottom slab from its unrotated planes 1 and 2
   float2 gx, gs, gI;
@@ -882,7 +928,7 @@ __global__ void __launch_bounds__(256, 3) k_quad_rot_column2(int nf, int nx, int
                      pl);
     gx = xd; gs = sd; gI = In;
   }
-  reinterpret_cast<float2 *>(I_top)[g] = gI;
+  reinterpret_cast<float2 *>(I_top)[g + plane * blockIdx.y] = gI;
 }
 
 // save_intensity (rt_patch_mod.f90:4151-4208): ie(f) = <2h nu^5/(c^3 AA) I>_xy, in
@@ -893,6 +939,7 @@ __global__ void k_save_partial(int nf, int ncol, const double *nu, const TI *I_t
   __shared__ double acc[8][33];
   const int f = blockIdx.x * 32 + threadIdx.x;
   const int nparts = gridDim.y;
+  I_top += (size_t)nf * ncol * blockIdx.z;      // one ray's plane
   double s = 0.0;
   if (f < nf) {
     const double conv = 2.0 * 6.626176e-27 / (2.99792458e10 * 2.99792458e10 * 2.99792458e10 * 1e8);
@@ -905,16 +952,36 @@ __global__ void k_save_partial(int nf, int ncol, const double *nu, const TI *I_t
   if (threadIdx.y == 0 && f < nf) {
     double t = 0.0;
     for (int k = 0; k < (int)blockDim.y; k++) t += acc[k][threadIdx.x];
-    part[(size_t)blockIdx.y * nf + f] = t;
+    part[((size_t)blockIdx.z * nparts + blockIdx.y) * nf + f] = t;
   }
 }
 
+// The partials in their order, eight loads in flight at a time (one by one the 148
+// loads' latencies added up to 16 us a ray); grid.y the rays.
 __global__ void k_save_final(int nf, int ncol, int nparts, const double *part, float *ie) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nf) return;
+  part += (size_t)nparts * nf * blockIdx.y + f;
   double t = 0.0;
-  for (int p = 0; p < nparts; p++) t += part[(size_t)p * nf + f];
-  ie[f] = (float)t / (float)ncol;
+  int p = 0;
+  for (; p + 8 <= nparts; p += 8) {
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = part[(size_t)(p + k) * nf];
+#pragma unroll
+    for (int k = 0; k < 8; k++) t += v[k];
+  }
+  for (; p < nparts; p++) t += part[(size_t)p * nf];
+  ie[f + (size_t)nf * blockIdx.y] = (float)t / (float)ncol;
+}
+
+// flux = 2 pi sum_mu wmu ie (rt_patch_mod.f90:4193-4200); w: 2 pi wmu in real(4)
+__global__ void k_flux(int nf, int nray, const float *w, const float *ie, float *flux) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= nf) return;
+  float v = 0.0f;
+  for (int r = 0; r < nray; r++) v = fmaf(w[r], ie[f + (size_t)nf * r], v);
+  flux[f] = v;
 }
 
 // copy the transfer units of a slab's planes into its FP64 work array (plain path)
