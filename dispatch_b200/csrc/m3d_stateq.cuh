@@ -5,8 +5,10 @@
 // partial pivoting) and the population update (update_populations :439-732);
 // then Ng's accumulation and extrapolation in ln b (SRC/ng_mod.f90:241-390).
 //
-// One warp owns one cell at a time and keeps the cell's rate matrix (column
-// major, n <= 64) and its vectors in shared memory.  Every elimination step
+// A team of threads owns one cell at a time and assembles the cell's rate matrix
+// (column major, n <= 64) and its vectors in shared memory.  lineq_no_pivot then takes
+// one matrix row per thread in registers (se_solve_rows); the pivoting solvers, and
+// lineq_no_pivot under M3D_SE_WARP, work in shared memory with one warp.  Every elimination step
 // updates each matrix element once, so spreading a step's elements over the
 // lanes performs exactly the roundings of the sequential loops; the
 // substitutions that a row-wise loop orders differently from a column-wise one
@@ -74,7 +76,8 @@ struct SeWarpBest {
 // ---- classic_col helpers (atom_mod.f90:2362-2467) ------------------------------
 // The Fortran tables are default-real literals: their single-precision values
 // enter the double arithmetic.
-__device__ __forceinline__ double se_expin(double x) {
+// ex = exp(-x)
+__device__ __forceinline__ double se_expin(double x, double ex) {
   const float a0 = -44178.5471728217f, a1 = 57721.7247139444f, a2 = 9938.31388962037f, a3 = 1842.11088668000f,
               a4 = 101.093806161906f, a5 = 5.03416184097568f;
   const float b0 = 76537.3323337614f, b1 = 32597.1881290275f, b2 = 6106.10794245759f, b3 = 635.419418378382f,
@@ -87,11 +90,17 @@ __device__ __forceinline__ double se_expin(double x) {
               e4 = -1298.85688746484f, e5 = -545.374158883133f, e6 = -5.66575206533869f;
   const float f0 = 28.6271060422192f, f1 = 292.310039388533f, f2 = 1332.78537748257f, f3 = 2777.61949509163f,
               f4 = 2404.01713225909f, f5 = 631.657483280800f;
-  const double ex = exp(-x);
   if (x > 4) {
-    return (ex + ex * ((double)e0 + ((double)e1 + ((double)e2 + ((double)e3 + ((double)e4 + ((double)e5 + (double)e6 / x) / x) / x) / x) / x) / x) /
-                     (x + (double)f0 + ((double)f1 + ((double)f2 + ((double)f3 + ((double)f4 + (double)f5 / x) / x) / x) / x) / x)) /
-           x;
+    // the nested quotients by x as one reciprocal and Horner steps (14 divisions left
+    // the collision rates a third of the update's time)
+    const double r = 1.0 / x;
+    double p = fma((double)e6, r, (double)e5), q = fma((double)f5, r, (double)f4);
+    p = fma(p, r, (double)e4); q = fma(q, r, (double)f3);
+    p = fma(p, r, (double)e3); q = fma(q, r, (double)f2);
+    p = fma(p, r, (double)e2); q = fma(q, r, (double)f1);
+    p = fma(p, r, (double)e1); q = fma(q, r, x + (double)f0);
+    p = fma(p, r, (double)e0);
+    return fma(ex, p / q, ex) * r;
   } else if (x > 1) {
     return ex * ((double)c6 + ((double)c5 + ((double)c4 + ((double)c3 + ((double)c2 + ((double)c1 + (double)c0 * x) * x) * x) * x) * x) * x) /
            ((double)d5 + ((double)d4 + ((double)d3 + ((double)d2 + ((double)d1 + ((double)d0 + x) * x) * x) * x) * x) * x);
@@ -182,9 +191,9 @@ __device__ __forceinline__ void se_col_rates(const SeAtomDev &A, const SeColCell
     v = w.seaton * fac * tmp / u0 * ex;
     v = v * A.cbfesc;
   } else if (!cont && kind == SE_COL_REGEMORTER) {
-    const double tmp = fmax((double)0.2f * ex, sqr3_2pi * se_expin(u0));
+    const double tmp = fmax((double)0.2f * ex, sqr3_2pi * se_expin(u0, ex));
     v = w.regemorter * f * tmp / dev;
-    v = fmax(v, w.allen * A.upsilon_floor * ex / A.g[i]);
+    v = fmax(v, A.upsilon_floor != 0 ? w.allen * A.upsilon_floor * ex / A.g[i] : 0.0);
     v = v * A.cbbesc;
   }
   if (v != 0) v = v * A.colscale;
@@ -343,7 +352,7 @@ __global__ void k_collision_rates(SeAtomDev A, SeCells C, double *__restrict__ c
 // a(i,j) = W[i + n*j]; e is the right-hand side, the solution on return.
 
 // A cell's team: TEAM threads share its matrix, one warp (TEAM = 32) or a whole
-// block of 64 or 128 threads, whose barriers are then the block's.
+// block of 64 threads, whose barriers are then the block's.
 template <int TEAM>
 __device__ __forceinline__ void team_sync() {
   if (TEAM == 32) __syncwarp();
@@ -371,8 +380,9 @@ __device__ __forceinline__ double se_elim(double aij, double l, double akj) {
 // the columns into G groups.  l(i) stays in a register and four columns' loads
 // precede their stores, so the FP64 chains of a lane overlap.  Every element takes
 // its one update per step, so the roundings are the sequential loop's.
-template <bool SKIP, int TEAM = 32>
+template <bool SKIP>
 __device__ __forceinline__ void se_elim_step(double *W, double *lstore, int n, int k, int lane) {
+  constexpr int TEAM = 32;
   const int m = n - k - 1;
   const double pk = W[k + n * k];
   const int G = m >= TEAM ? 1 : TEAM / m;
@@ -417,15 +427,14 @@ __device__ __forceinline__ void se_elim_step(double *W, double *lstore, int n, i
   team_sync<TEAM>();
 }
 
-// lineq_no_pivot (op_math_mod.f90:420-449)
-template <int TEAM = 32>
+// lineq_no_pivot (op_math_mod.f90:420-449) in shared memory
 __device__ __forceinline__ void se_solve_no_pivot(double *W, double *e, int n, int lane) {
-  for (int k = 0; k < n - 1; k++) se_elim_step<true, TEAM>(W, W + n * k, n, k, lane);
+  for (int k = 0; k < n - 1; k++) se_elim_step<true>(W, W + n * k, n, k, lane);
   // forward substitution: per row the terms arrive in ascending j, as in the row loop
   for (int j = 0; j < n - 1; j++) {
     const double ej = e[j];
-    for (int i = j + 1 + lane; i < n; i += TEAM) e[i] = e[i] - W[i + n * j] * ej;
-    team_sync<TEAM>();
+    for (int i = j + 1 + lane; i < n; i += 32) e[i] = e[i] - W[i + n * j] * ej;
+    __syncwarp();
   }
   // back substitution: the row loop adds its terms in ascending j, an order no
   // column sweep reproduces, so one lane runs it
@@ -434,6 +443,99 @@ __device__ __forceinline__ void se_solve_no_pivot(double *W, double *e, int n, i
       double t = e[i];
       for (int j = i + 1; j < n; j++) t = t - W[i + n * j] * e[j];
       e[i] = t / W[i + n * i];
+    }
+  }
+  __syncwarp();
+}
+
+// lineq_no_pivot with a thread per row, the row in registers: a[j] is the row's element
+// of column k + j, so that the step's loop runs over fixed registers and its results
+// move one place down.  Row k is final at step k; its thread writes it to shared memory
+// (U, rows of LD doubles, element j of row k at column k + j), where every other row
+// reads it back by broadcast, two elements a load.  The rows shrink by eight registers
+// every eight steps.  Where the start kept the matrix in shared memory, each update
+// cost two shared loads and a store (88 % of the 21-level update's 8.2 ms a 262144
+// cells, and 5 to 7 cells an SM at 61 levels).
+//
+// A row whose pivot element vanishes is updated like the others, where the
+// shared-memory form skips it: a - l 0 is a for every finite l (but for the sign of a
+// zero, which reaches no finite result), and a row with an infinite or undefined l
+// takes the skipping form.
+template <int N, int TEAM, int R>
+struct SeRowSteps {
+  static __device__ __forceinline__ void run(double (&a)[N], double &ei, double *U, double *es, int n, int row,
+                                             int k0) {
+    constexpr int LD = N + 2;
+    const int kend = min(k0 + 8, n - 1);
+    for (int k = k0; k < kend; k++) {
+      double *u = U + LD * k;
+      if (row == k) {
+#pragma unroll
+        for (int j = 0; j < R; j += 2) *reinterpret_cast<double2 *>(u + j) = make_double2(a[j], a[j + 1]);
+        es[k] = ei;
+      }
+      team_sync<TEAM>();
+      if (row > k) {
+        const double l = a[0] / u[0];
+        ei = ei - l * es[k];
+        if (fabs(l) <= DBL_MAX) {
+#pragma unroll
+          for (int j = 0; j < R; j += 2) {
+            const double2 p = *reinterpret_cast<const double2 *>(u + j);
+            if (j > 0) a[j - 1] = a[j] - l * p.x;
+            a[j] = a[j + 1] - l * p.y;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < R; j += 2) {
+            const double2 p = *reinterpret_cast<const double2 *>(u + j);
+            if (j > 0) a[j - 1] = p.x != 0 ? a[j] - l * p.x : a[j];
+            a[j] = p.y != 0 ? a[j + 1] - l * p.y : a[j + 1];
+          }
+        }
+      }
+    }
+    if constexpr (R > 8)
+      if (kend < n - 1) SeRowSteps<N, TEAM, R - 8>::run(a, ei, U, es, n, row, kend);
+  }
+};
+
+// W(i, j) b_j n*_j of row i (the conservation row: b_j n*_j alone) is formed as the row
+// is read; es: the right-hand side and the solution; U overlays W.
+template <int N, int TEAM>
+__device__ __forceinline__ void se_solve_rows(const double *W, int ldw, double *U, double *es, const double *bl,
+                                              const double *ns, int pos, double totn, int n, int row) {
+  constexpr int LD = N + 2;
+  double a[N];
+  double ei = row == pos ? totn : 0.0;
+#pragma unroll
+  for (int j = 0; j < N; j++) {
+    a[j] = 0.0;
+    if (row < n && j < n) a[j] = row == pos ? bl[j] * ns[j] : (W[row + ldw * j] * bl[j]) * ns[j];
+  }
+  team_sync<TEAM>();
+  SeRowSteps<N, TEAM, N>::run(a, ei, U, es, n, row, 0);
+  if (row == n - 1) {
+    // the last row's one element left
+    U[LD * (n - 1)] = a[0];
+    es[n - 1] = ei;
+  }
+  team_sync<TEAM>();
+  // Back substitution: the row loop adds its terms in ascending j, so row i's sum starts
+  // with the value found last.  Each value's products with its column are formed by all
+  // lanes as it is found (in place in U); the sums follow in order, one at a time.
+  if (TEAM == 32 || row < 32) {
+    double x = 0;
+    for (int i = n - 1; i >= 0; i--) {
+      const double *u = U + LD * i;
+      double t = es[i];
+      if (i + 1 < n) t = t - u[1] * x;
+#pragma unroll 8
+      for (int j = 2; j < n - i; j++) t = t - u[j];
+      x = t / u[0];
+      if (row == 0) es[i] = x;
+      for (int r = row; r <= i - 2; r += 32) U[LD * r + i - r] = U[LD * r + i - r] * x;
+      __syncwarp();
     }
   }
   team_sync<TEAM>();
@@ -582,23 +684,43 @@ __device__ __forceinline__ void se_solve_partial(double *W, double *e, int n, in
   }
 }
 
-// shared memory of one warp, in doubles (plus n ints for lineq's column order)
-__host__ __device__ inline size_t se_warp_doubles(int n) { return (size_t)n * n + 4 * (size_t)n + (size_t)(n + 1) / 2; }
+// Shared memory of one team, in doubles: the matrix (and with rows in registers the
+// factor's rows over it), four vectors, and n ints for lineq's column order.  The
+// register form's columns start an odd number of doubles apart, so that a column a lane
+// sums (the diagonal) is read without bank conflicts.
+__host__ __device__ inline int se_ldw(int n, int N) { return N > 0 ? (n | 1) : n; }
+__host__ __device__ inline size_t se_matrix_doubles(int n, int N) {
+  const size_t w = (size_t)se_ldw(n, N) * n, u = (size_t)N * (N + 2);
+  return ((w > u ? w : u) + 1) & ~(size_t)1;
+}
+__host__ __device__ inline size_t se_team_doubles(int n, int N) {
+  return (se_matrix_doubles(n, N) + 4 * (size_t)n + (size_t)(n + 1) / 2 + 1) & ~(size_t)1;
+}
+
+// blocks per SM that the register form's rows leave room for: its N doubles a thread
+// and some fifty registers beside them; the general collision forms take what they need
+__host__ __device__ constexpr int se_threads(int TEAM, int N) { return N == 0 ? 128 : TEAM == 64 ? 64 : 128; }
+__host__ __device__ constexpr int se_min_blocks(int CM, int N) {
+  return N == 0 ? (CM == 2 ? 2 : 4) : CM == 2 ? 1 : N <= 16 ? 6 : N <= 24 ? 5 : N <= 32 ? 4 : N <= 48 ? 7 : 6;
+}
 
 // update_populations over all cells: warps stride over the cells in ascending order
 // CM 0: collision rates read from C.cup (or none); 1: formed here, electron
 // recipes only; 2: formed here, any recipes and records.  The host picks the
 // least general form, which keeps the common ones' register use down.
-template <int CM, int TEAM = 32>
-__global__ void k_stateq_update(SeAtomDev A, SeParams P, SeCells C, SeWarpBest *__restrict__ wbest,
+// N: lineq_no_pivot with a thread per row of up to N registers (se_solve_rows); 0: the
+// solvers in shared memory, one warp.
+template <int CM, int TEAM, int N>
+__global__ void __launch_bounds__(se_threads(TEAM, N), se_min_blocks(CM, N)) k_stateq_update(SeAtomDev A, SeParams P, SeCells C, SeWarpBest *__restrict__ wbest,
                                 double *__restrict__ lvl_val, long long *__restrict__ lvl_cell,
                                 unsigned long long *__restrict__ counts, long long *__restrict__ nonfinite) {
-  extern __shared__ double se_smem[];
+  extern __shared__ __align__(16) double se_smem[];
   // a team of TEAM threads per cell: a warp (several teams per block), or the block
   const int n = A.n, lane = TEAM == 32 ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
   const int wib = TEAM == 32 ? (int)(threadIdx.x >> 5) : 0;
-  double *W = se_smem + se_warp_doubles(n) * wib;
-  double *bl = W + n * n, *ns = bl + n, *e = ns + n, *q = e + n;
+  const int ldw = se_ldw(n, N);
+  double *W = se_smem + se_team_doubles(n, N) * wib;
+  double *bl = W + se_matrix_doubles(n, N), *ns = bl + n, *e = ns + n, *q = e + n;
   int *icol = (int *)(q + n);
   const int tpb = TEAM == 32 ? (int)(blockDim.x >> 5) : 1;  // teams per block
   const int nwarp = gridDim.x * tpb;
@@ -626,21 +748,32 @@ __global__ void k_stateq_update(SeAtomDev A, SeParams P, SeCells C, SeWarpBest *
       ns[k] = C.nstar[(size_t)c + (size_t)ncell * k];
       e[k] = 0;
     }
-    for (int idx = lane; idx < n * n; idx += TEAM) W[idx] = 0;
+    for (int idx = lane; idx < ldw * n; idx += TEAM) W[idx] = 0;
     team_sync<TEAM>();
-    // radiative rates, round by round
+    // radiative rates, round by round; a lane's first four transitions' rates are
+    // loaded together
     for (int r = 0; r < A.nround; r++) {
-      for (int t = A.round_off[r] + lane; t < A.round_off[r + 1]; t += TEAM) {
+      const int t0 = A.round_off[r] + lane, t1 = A.round_off[r + 1];
+      constexpr int NP = 4;
+      float pth[NP], pdv[NP];
+#pragma unroll
+      for (int q = 0; q < NP; q++) {
+        const int t = t0 + q * TEAM;
+        const size_t o = (size_t)c + (size_t)ncell * (t < t1 ? A.order[t] : 0);
+        pth[q] = t < t1 ? C.gij[o] : 0.0f;
+        pdv[q] = t < t1 ? C.gji[o] : 0.0f;
+      }
+      auto add = [&](int t, float fth, float fdv) {
         const int kr = A.order[t];
         const int i = A.ti[kr], j = A.tj[kr];
         if ((A.ev[j] - A.ev[i]) * ekt > A.cut_x) {
           const double cut_rate = kr < A.nline ? A.Aji[kr] : A.bf_cut_rate;
-          W[i + n * j] = W[i + n * j] + cut_rate;
-          W[j + n * i] = W[j + n * i] + cut_rate * ns[j] / ns[i];
-          continue;
+          W[i + ldw * j] = W[i + ldw * j] + cut_rate;
+          W[j + ldw * i] = W[j + ldw * i] + cut_rate * ns[j] / ns[i];
+          return;
         }
-        const double th = (double)C.gij[(size_t)c + (size_t)ncell * kr];
-        const double dv = (double)C.gji[(size_t)c + (size_t)ncell * kr];
+        const double th = (double)fth;
+        const double dv = (double)fdv;
         double r_up, r_down;
         if (kr < A.nline) {
           const double g_ij = A.g[i] / A.g[j];
@@ -656,8 +789,15 @@ __global__ void k_stateq_update(SeAtomDev A, SeParams P, SeCells C, SeWarpBest *
           r_up = th;
           r_down = dv;
         }
-        W[j + n * i] = W[j + n * i] + r_up;
-        W[i + n * j] = W[i + n * j] + r_down;
+        W[j + ldw * i] = W[j + ldw * i] + r_up;
+        W[i + ldw * j] = W[i + ldw * j] + r_down;
+      };
+#pragma unroll
+      for (int q = 0; q < NP; q++)
+        if (t0 + q * TEAM < t1) add(t0 + q * TEAM, pth[q], pdv[q]);
+      for (int t = t0 + NP * TEAM; t < t1; t += TEAM) {
+        const size_t o = (size_t)c + (size_t)ncell * A.order[t];
+        add(t, C.gij[o], C.gji[o]);
       }
       team_sync<TEAM>();
     }
@@ -713,7 +853,8 @@ __global__ void k_stateq_update(SeAtomDev A, SeParams P, SeCells C, SeWarpBest *
               cv = cv + (type == 2 ? up : dn);
             }
           }
-          W[A.el_w[e]] = W[A.el_w[e]] + cv * P.cswitch;
+          const int w = A.el_w[e] + (ldw - n) * (A.el_w[e] / n);
+          W[w] = W[w] + cv * P.cswitch;
         }
       } else {
         for (int p = lane; p < A.ncol; p += TEAM) {
@@ -731,8 +872,8 @@ __global__ void k_stateq_update(SeAtomDev A, SeParams P, SeCells C, SeWarpBest *
             cu = cu + uh;
             cd = cd + uh * nij;
           }
-          W[j + n * i] = W[j + n * i] + cu * P.cswitch;
-          W[i + n * j] = W[i + n * j] + cd * P.cswitch;
+          W[j + ldw * i] = W[j + ldw * i] + cu * P.cswitch;
+          W[i + ldw * j] = W[i + ldw * j] + cd * P.cswitch;
         }
       }
       team_sync<TEAM>();
@@ -740,32 +881,38 @@ __global__ void k_stateq_update(SeAtomDev A, SeParams P, SeCells C, SeWarpBest *
     // diagonal = -(column sum), each lane one column
     for (int i = lane; i < n; i += TEAM) {
       double s = 0;
-      for (int k = 0; k < n; k++) s = s + W[k + n * i];
-      W[i + n * i] = -s;
+      for (int k = 0; k < n; k++) s = s + W[k + ldw * i];
+      W[i + ldw * i] = -s;
     }
-    // the conservation row: the first level of largest b n*
-    int pos = 0;
+    // the conservation row: the first level of largest b n*.  A sequential scan from
+    // level 0 that moves on a strict increase keeps level 0 if its value is undefined
+    // and passes over the other undefined ones.
+    int pos;
     {
-      double bst = bl[0] * ns[0];
-      for (int k = 1; k < n; k++) {
+      const int wl = threadIdx.x & 31;
+      double bst = -INFINITY;
+      pos = -1;
+      for (int k = wl; k < n; k += 32) {
         const double v = bl[k] * ns[k];
-        if (v > bst) { bst = v; pos = k; }
+        if (v == v && (pos < 0 || v > bst)) { bst = v; pos = k; }
       }
+      warp_argmax(bst, pos);
+      const double v0 = bl[0] * ns[0];
+      if (v0 != v0 || pos < 0) pos = 0;
     }
     team_sync<TEAM>();
-    for (int idx = lane; idx < n * n; idx += TEAM) {
-      const int i = idx % n, j = idx / n;
-      W[idx] = (i == pos) ? bl[j] * ns[j] : (W[idx] * bl[j]) * ns[j];
-    }
-    if (lane == 0) e[pos] = totn;
-    team_sync<TEAM>();
-
-    if constexpr (TEAM == 32) {
+    if constexpr (N > 0) {
+      se_solve_rows<N, TEAM>(W, ldw, W, e, bl, ns, pos, totn, n, lane);
+    } else {
+      for (int idx = lane; idx < n * n; idx += TEAM) {
+        const int i = idx % n, j = idx / n;
+        W[idx] = (i == pos) ? bl[j] * ns[j] : (W[idx] * bl[j]) * ns[j];
+      }
+      if (lane == 0) e[pos] = totn;
+      team_sync<TEAM>();
       if (P.solver == 1) se_solve_lineq(W, e, q, icol, n, lane);
       else if (P.solver == 2) se_solve_partial(W, e, n, lane);
       else se_solve_no_pivot(W, e, n, lane);
-    } else {
-      se_solve_no_pivot<TEAM>(W, e, n, lane);  // the host sends only lineq_no_pivot to larger teams
     }
 
     bool finite = true;
@@ -788,6 +935,7 @@ __global__ void k_stateq_update(SeAtomDev A, SeParams P, SeCells C, SeWarpBest *
     }
     team_sync<TEAM>();
     double sum = 0;
+#pragma unroll 4
     for (int k = 0; k < n; k++) sum = sum + bl[k] * ns[k];
     const double norm = totn / sum;
     double wv = -1.0;
@@ -830,43 +978,50 @@ __global__ void k_stateq_update(SeAtomDev A, SeParams P, SeCells C, SeWarpBest *
   }
 }
 
-// one block: the largest change over the warps' partials, ties to the first cell
+// The largest change over the teams' partials, ties to the first cell: block 0 the
+// overall one, block 1 + k level k's.  The order does not matter to the result, so each
+// thread takes every 256th partial and the block reduces them (one thread a level over
+// all partials took 0.62 ms).
 __global__ void k_stateq_finish(int nwarp, int n, const SeWarpBest *__restrict__ wbest,
                                 const double *__restrict__ lvl_val, const long long *__restrict__ lvl_cell,
                                 SeWarpBest *__restrict__ out_best, double *__restrict__ out_lvl) {
-  __shared__ SeWarpBest sb[256];
-  SeWarpBest b;
-  b.maxerr_abs = 0;
-  b.maxerr = 0;
-  b.cell = -1;
-  b.level = -1;
-  b.pad = 0;
-  for (int w = threadIdx.x; w < nwarp; w += blockDim.x) {
-    const SeWarpBest o = wbest[w];
-    if (o.cell >= 0 && (b.cell < 0 || o.maxerr_abs > b.maxerr_abs || (o.maxerr_abs == b.maxerr_abs && o.cell < b.cell)))
-      b = o;
-  }
-  sb[threadIdx.x] = b;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    SeWarpBest r = sb[0];
-    for (int t = 1; t < (int)blockDim.x; t++) {
-      const SeWarpBest o = sb[t];
+  if (blockIdx.x == 0) {
+    __shared__ SeWarpBest sb[256];
+    SeWarpBest b;
+    b.maxerr_abs = 0;
+    b.maxerr = 0;
+    b.cell = -1;
+    b.level = -1;
+    b.pad = 0;
+    auto take = [](SeWarpBest &r, const SeWarpBest &o) {
       if (o.cell >= 0 && (r.cell < 0 || o.maxerr_abs > r.maxerr_abs || (o.maxerr_abs == r.maxerr_abs && o.cell < r.cell)))
         r = o;
+    };
+    for (int w = threadIdx.x; w < nwarp; w += blockDim.x) take(b, wbest[w]);
+    sb[threadIdx.x] = b;
+    for (int h = blockDim.x / 2; h > 0; h /= 2) {
+      __syncthreads();
+      if ((int)threadIdx.x < h) take(sb[threadIdx.x], sb[threadIdx.x + h]);
     }
-    *out_best = r;
+    if (threadIdx.x == 0) *out_best = sb[0];
+    return;
   }
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    double v = 0;
-    long long cc = -1;
-    for (int w = 0; w < nwarp; w++) {
-      const long long oc = lvl_cell[(size_t)w * n + k];
-      const double ov = lvl_val[(size_t)w * n + k];
-      if (oc >= 0 && (cc < 0 || fabs(ov) > fabs(v) || (fabs(ov) == fabs(v) && oc < cc))) { v = ov; cc = oc; }
-    }
-    out_lvl[k] = v;
+  __shared__ double sv[256];
+  __shared__ long long sc[256];
+  const int k = blockIdx.x - 1;
+  double v = 0;
+  long long cc = -1;
+  auto take = [](double &rv, long long &rc, double ov, long long oc) {
+    if (oc >= 0 && (rc < 0 || fabs(ov) > fabs(rv) || (fabs(ov) == fabs(rv) && oc < rc))) { rv = ov; rc = oc; }
+  };
+  for (int w = threadIdx.x; w < nwarp; w += blockDim.x) take(v, cc, lvl_val[(size_t)w * n + k], lvl_cell[(size_t)w * n + k]);
+  sv[threadIdx.x] = v;
+  sc[threadIdx.x] = cc;
+  for (int h = blockDim.x / 2; h > 0; h /= 2) {
+    __syncthreads();
+    if ((int)threadIdx.x < h) take(sv[threadIdx.x], sc[threadIdx.x], sv[threadIdx.x + h], sc[threadIdx.x + h]);
   }
+  if (threadIdx.x == 0) out_lvl[k] = sv[0];
 }
 
 // ---- Ng acceleration (ng_mod.f90:241-390) ---------------------------------------

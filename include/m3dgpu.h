@@ -711,16 +711,16 @@ int m3d_collision_rates(const m3d_atom_t *atom, int ncell, const double *e_kT, c
  * filter.  lvlerr (nlevel, host) and res (host) receive the convergence record.
  * A cell whose solution is not finite keeps its b, and the call returns
  * M3D_ENONFINITE with res->nonfinite_cell set (the reference stops the run there).
- * Each cell is solved by a team of threads sharing its matrix: one warp, or for
- * lineq_no_pivot a block of 64 or 128 threads when that keeps more threads resident
- * (large atoms); every element takes the same operations in the same order either
- * way.  M3D_SE_WARP keeps one warp per cell. */
+ * Each cell is solved by a team of threads: one warp, or for lineq_no_pivot and more
+ * than 32 levels a block of 64 threads, a thread per matrix row; every element takes
+ * the same operations in the same order either way.  M3D_SE_WARP keeps one warp per
+ * cell. */
 int m3d_stateq_update(const m3d_atom_t *atom, const m3d_se_params_t *par, int ncell, double *b,
                       const double *nstar, const double *totn, const double *e_kT,
                       const m3d_col_cells_t *cells, const float *gamma_ij, const float *gamma_ji,
                       const double *cup, double *lvlerr, m3d_se_result_t *res, unsigned flags);
 
-/* Threads per cell of this thread context's last m3d_stateq_update (32, 64 or 128;
+/* Threads per cell of this thread context's last m3d_stateq_update (32 or 64;
  * 0 before the first).  Diagnostic. */
 int m3d_stateq_team(void);
 
