@@ -25,6 +25,10 @@ constexpr int SE_NMAX = 64;
 constexpr int SE_COL_REGEMORTER = 1, SE_COL_SEATON = 2;
 constexpr int SE_COLH_DRAWIN = 1, SE_COLH_TAKEDA = 2;
 
+// A bound pair under van Regemorter's recipe: its energy, f/dev, 1-in-16-bytes beside
+// its levels
+struct __align__(16) SePair { double dev, fdev; int i, j; double gi; };
+
 // Atom tables in device memory.  Transitions are listed by round: the
 // transitions of one round touch pairwise different matrix elements, and a
 // pair's transitions fall in successive rounds in their original order, so
@@ -40,6 +44,11 @@ struct SeAtomDev {
   const int *ci, *cj, *ckind;  // [ncol]
   const float *cfac;           // [ncol]
   const int *chkind;           // [ncol] hydrogen recipes, or null: none
+  // the pairs again, sorted for the electron recipes alone: first the nreg bound ones
+  // under van Regemorter's, each a record; then the others' indices, rest[ncol - nreg]
+  int nreg;
+  const SePair *reg;
+  const int *rest;
   double fmin, cbbesc, cbfesc, colscale, upsilon_floor, cut_x, bf_cut_rate;
   double drawin, cbbhsc, cbfhsc;
   // gencol's records (atom_mod.f90:2223-2360) and, with records, the matrix
@@ -76,40 +85,25 @@ struct SeWarpBest {
 // ---- classic_col helpers (atom_mod.f90:2362-2467) ------------------------------
 // The Fortran tables are default-real literals: their single-precision values
 // enter the double arithmetic.
-// ex = exp(-x)
-__device__ __forceinline__ double se_expin(double x, double ex) {
-  const float a0 = -44178.5471728217f, a1 = 57721.7247139444f, a2 = 9938.31388962037f, a3 = 1842.11088668000f,
-              a4 = 101.093806161906f, a5 = 5.03416184097568f;
-  const float b0 = 76537.3323337614f, b1 = 32597.1881290275f, b2 = 6106.10794245759f, b3 = 635.419418378382f,
-              b4 = 37.2298352833327f;
-  const float c0 = 4.65627107975096e-7f, c1 = .999979577051595f, c2 = 9.04161556946329f, c3 = 24.3784088791317f,
-              c4 = 23.0192559391333f, c5 = 6.90522522784444f, c6 = .430967839469389f;
-  const float d0 = 10.0411643829054f, d1 = 32.4264210695138f, d2 = 41.2807841891424f, d3 = 20.4494785013794f,
-              d4 = 3.31909213593302f, d5 = .103400130404874f;
-  const float e0 = -.999999999998447f, e1 = -26.6271060431811f, e2 = -241.055827097015f, e3 = -895.927957772937f,
-              e4 = -1298.85688746484f, e5 = -545.374158883133f, e6 = -5.66575206533869f;
-  const float f0 = 28.6271060422192f, f1 = 292.310039388533f, f2 = 1332.78537748257f, f3 = 2777.61949509163f,
-              f4 = 2404.01713225909f, f5 = 631.657483280800f;
-  if (x > 4) {
-    // the nested quotients by x as one reciprocal and Horner steps (14 divisions left
-    // the collision rates a third of the update's time)
-    const double r = 1.0 / x;
-    double p = fma((double)e6, r, (double)e5), q = fma((double)f5, r, (double)f4);
-    p = fma(p, r, (double)e4); q = fma(q, r, (double)f3);
-    p = fma(p, r, (double)e3); q = fma(q, r, (double)f2);
-    p = fma(p, r, (double)e2); q = fma(q, r, (double)f1);
-    p = fma(p, r, (double)e1); q = fma(q, r, x + (double)f0);
-    p = fma(p, r, (double)e0);
-    return fma(ex, p / q, ex) * r;
-  } else if (x > 1) {
-    return ex * ((double)c6 + ((double)c5 + ((double)c4 + ((double)c3 + ((double)c2 + ((double)c1 + (double)c0 * x) * x) * x) * x) * x) * x) /
-           ((double)d5 + ((double)d4 + ((double)d3 + ((double)d2 + ((double)d1 + ((double)d0 + x) * x) * x) * x) * x) * x);
-  } else if (x > 0) {
-    return ((double)a0 + ((double)a1 + ((double)a2 + ((double)a3 + ((double)a4 + (double)a5 * x) * x) * x) * x) * x) /
-               ((double)b0 + ((double)b1 + ((double)b2 + ((double)b3 + ((double)b4 + x) * x) * x) * x) * x) -
-           log(x);
+// van Regemorter's Gaunt factor, the larger of 0.2 e^-u and sqrt(3)/(2 pi) E1(u), with
+// E1 of expin (atom_mod.f90:2362-2397).  e^u E1(u) falls with u and is 0.596 at 1, where
+// 0.276 times it is below 0.2 by a fifth (the fits' errors are under 1e-5): above 1 the
+// first term is the larger and E1's two other fits are never needed.  ex = e^-u.
+__device__ __forceinline__ double se_regemorter_g(double u, double ex) {
+  const double sqr3_2pi = (sqrt(3.0) / 2.0) / 3.14159265359;
+  const double lo = (double)0.2f * ex;
+  if (u > 1) return lo;
+  double e1 = 0.0;
+  if (u > 0) {
+    const float a0 = -44178.5471728217f, a1 = 57721.7247139444f, a2 = 9938.31388962037f, a3 = 1842.11088668000f,
+                a4 = 101.093806161906f, a5 = 5.03416184097568f;
+    const float b0 = 76537.3323337614f, b1 = 32597.1881290275f, b2 = 6106.10794245759f, b3 = 635.419418378382f,
+                b4 = 37.2298352833327f;
+    e1 = ((double)a0 + ((double)a1 + ((double)a2 + ((double)a3 + ((double)a4 + (double)a5 * u) * u) * u) * u) * u) /
+             ((double)b0 + ((double)b1 + ((double)b2 + ((double)b3 + ((double)b4 + u) * u) * u) * u) * u) -
+         log(u);
   }
-  return 0.0;
+  return fmax(lo, sqr3_2pi * e1);
 }
 
 __constant__ float se_gaunt_a1[6] = {1.078e00f, 1.0926e0f, 1.0983e0f, 1.0954e0f, 1.0912e0f, 1.0925e0f};
@@ -160,13 +154,21 @@ __device__ __forceinline__ SeColCell se_col_cell(double temp, double ne, double 
   return w;
 }
 
+// van Regemorter's rate of a bound pair: f/dev its oscillator strength over its energy,
+// u0 = dev / kT, ex = e^-u0, gi the lower level's weight (before colscale)
+__device__ __forceinline__ double se_regemorter(const SeAtomDev &A, const SeColCell &w, double fdev, double ex,
+                                                double u0, double gi) {
+  double v = w.regemorter * fdev * se_regemorter_g(u0, ex);
+  v = fmax(v, A.upsilon_floor != 0 ? w.allen * A.upsilon_floor * ex / gi : 0.0);
+  return v * A.cbbesc;
+}
+
 // upward collision rates of pair p [1/s], colscale applied: ue by the pair's
 // electron recipe, uh by its hydrogen recipe (0 without one).  The electron mass
 // ame of the hydrogen recipes is a default-real literal (atom_mod.f90:220-222).
 template <bool HYD>
 __device__ __forceinline__ void se_col_rates(const SeAtomDev &A, const SeColCell &w, int p, double &ue,
                                              double &uh) {
-  const double sqr3_2pi = (sqrt(3.0) / 2.0) / 3.14159265359;
   const int i = A.ci[p], j = A.cj[p], kind = A.ckind[p];
   const int ioni = A.ion[i], ionj = A.ion[j];
   const bool cont = ionj > ioni;
@@ -191,10 +193,7 @@ __device__ __forceinline__ void se_col_rates(const SeAtomDev &A, const SeColCell
     v = w.seaton * fac * tmp / u0 * ex;
     v = v * A.cbfesc;
   } else if (!cont && kind == SE_COL_REGEMORTER) {
-    const double tmp = fmax((double)0.2f * ex, sqr3_2pi * se_expin(u0, ex));
-    v = w.regemorter * f * tmp / dev;
-    v = fmax(v, A.upsilon_floor != 0 ? w.allen * A.upsilon_floor * ex / A.g[i] : 0.0);
-    v = v * A.cbbesc;
+    v = se_regemorter(A, w, f / dev, ex, u0, A.g[i]);
   }
   if (v != 0) v = v * A.colscale;
   ue = v;
@@ -857,7 +856,21 @@ __global__ void __launch_bounds__(se_threads(TEAM, N), se_min_blocks(CM, N)) k_s
           W[w] = W[w] + cv * P.cswitch;
         }
       } else {
-        for (int p = lane; p < A.ncol; p += TEAM) {
+        // the electron recipes alone: the sorted pairs, so that a warp's lanes run one
+        // recipe and a pair's constants come in two loads
+        if (CM == 1)
+          for (int p = lane; p < A.nreg; p += TEAM) {
+            const SePair r = A.reg[p];
+            const double u0 = r.dev * ekt;
+            double ue = se_regemorter(A, cw, r.fdev, exp(-u0), u0, r.gi);
+            if (ue == 0) continue;
+            ue = ue * A.colscale;
+            const double nij = ns[r.i] / ns[r.j];
+            W[r.j + ldw * r.i] = W[r.j + ldw * r.i] + ue * P.cswitch;
+            W[r.i + ldw * r.j] = W[r.i + ldw * r.j] + (ue * nij) * P.cswitch;
+          }
+        for (int q = lane; q < (CM == 1 ? A.ncol - A.nreg : A.ncol); q += TEAM) {
+          const int p = CM == 1 ? A.rest[q] : q;
           double ue, uh;
           pair_rates(p, ue, uh);
           if (ue == 0 && uh == 0) continue;
