@@ -1278,19 +1278,24 @@ int launch_opacity(SynthIn &in, const double *v, const double *d_vr, int nray, b
   const size_t ncell = in.ncell;
   const int block = 256, warps = block / 32;
   const bool wins = in.nwin > 1;
-  const GridArgs *no_gw = nullptr;
   if (fp64) {
-    const size_t want = (ncell * in.nwin * nray + block - 1) / block;
-    const int grid = (int)std::min<size_t>(want, 148 * 8);
-    if (wins)
-      LAUNCH_S(M3D_STAGE_OPACITY, (k_lte_opacity_units_f64<32, true>), grid, block, 0, in.A, in.G, in.dnu,
-               (double *)dchi, (double *)dS, (const double2 *)g_ctx.d_tab64, in.d_Gw, in.nwin, d_vr, nray);
-    else if (nf == 32)
-      LAUNCH_S(M3D_STAGE_OPACITY, k_lte_opacity_units_f64<32>, grid, block, 0, in.A, in.G, in.dnu, (double *)dchi,
-               (double *)dS, (const double2 *)g_ctx.d_tab64, no_gw, 1, d_vr, nray);
-    else
-      LAUNCH_S(M3D_STAGE_OPACITY, k_lte_opacity_units_f64<0>, grid, block, 0, in.A, in.G, in.dnu, (double *)dchi,
-               (double *)dS, (const double2 *)g_ctx.d_tab64, no_gw, 1, d_vr, nray);
+    // 4 to 32 double registers a lane; windows above 32 take 2 to 32 lanes a cell
+    using F64Kernel = void (*)(AtmosDev, GridArgs, const double *, double *, double *, const double2 *,
+                               const GridArgs *, int, const double *, int, int, int *);
+    int P = 1;
+    while (32 * P < nf) P *= 2;
+    const F64Kernel k = wins      ? k_lte_opacity_units_f64<32, true>
+                        : nf <= 4 ? k_lte_opacity_units_f64<4>
+                        : nf <= 8 ? k_lte_opacity_units_f64<8>
+                        : nf <= 16 ? k_lte_opacity_units_f64<16>
+                                   : k_lte_opacity_units_f64<32>;
+    const size_t smem = QLG_NTAB * sizeof(double2);
+    CUDA_TRY(cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int *next;
+    TRY(unit_counter(&next));
+    const size_t cw = 32 / P, units = (ncell * nray + cw - 1) / cw * in.nwin;
+    LAUNCH_S(M3D_STAGE_OPACITY, k, (int)std::min<size_t>(units, (size_t)sm_count()), 512, smem, in.A, in.G, in.dnu,
+             (double *)dchi, (double *)dS, (const double2 *)g_ctx.d_tab64, in.d_Gw, in.nwin, d_vr, nray, P, next);
     return M3D_OK;
   }
   if (in.reach) {

@@ -519,11 +519,10 @@ __global__ void __launch_bounds__(lane_threads(NF), 1)
 
 // ---------------------------------------------------------------------------
 // The plain FP64 path of the same pass: the line opacity, the QLG-bot profile and
-// the transfer units all in double.  One lane per cell, chi_l of the window in
-// double registers, the general window form (per-point predicates) for every line.
-// The algorithm is the FP32 pass's step for step; what changes is the arithmetic:
+// the transfer units all in double.  The algorithm is the FP32 pass's step for step;
+// what changes is the arithmetic:
 //  * the tables TGX = 2^-u and TH2X = Z_0.2(u)(1+u)^2 are the fp64 values of
-//    qlg_init's formulas (not rounded to float), read from global memory;
+//    qlg_init's formulas (not rounded to float), 141 KB in shared memory;
 //  * the QLG-bot constants are the exact values the fitted float parameters stand
 //    for (1/pi, sqrt(ln2/pi), sqrt(ln2), 1/sqrt(pi)); the fit's own coefficients are
 //    the published digits;
@@ -549,12 +548,27 @@ __device__ __forceinline__ QlgCoef64 qlg_setup64(double gL, double D, double SQ,
   return c;
 }
 
-__device__ __forceinline__ double qlg_eval64(const double2 *tab, const QlgCoef64 &c, double x) {
-  const double xs = fabs(x) * c.ih;
-  const double u = xs * xs;
-  const double L = 1.0 / (1.0 + u);
-  const int ig = (int)lround(fmin(xs * 800.0, 9019.0));
-  const double2 gw = __ldg(tab + ig);
+// 1/d for 1 <= d <= 1e300 to an ulp: the approximate reciprocal (20 bits) and two Newton
+// steps, r + r (1 - d r), each of which squares the error
+__device__ __forceinline__ double rcp_newton64(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  r = fma(r, fma(-d, r, 1.0), r);
+  return fma(r, fma(-d, r, 1.0), r);
+}
+
+// the profile at abscissa x times ih, xs (either sign).  FAR: beyond the table, whose
+// last node's G and W are folded into p1 and gg.  BIG: 1 + xs^2 may exceed 1e300.
+template <bool FAR, bool BIG>
+__device__ __forceinline__ double qlg_eval64(const double2 *tab, const QlgCoef64 &c, double xs, double p1, double gg) {
+  const double d = fma(xs, xs, 1.0);
+  const double L = BIG ? 1.0 / d : rcp_newton64(d);
+  if (FAR) return fma(L, fma(L, p1, c.bL), gg);
+  // the snapped node nint(y), halves up: floor(RZ(y + 0.5)), read from the low word of
+  // RZ(that + 2^52), as qlg_node does in single
+  const double y = fmin(fabs(xs) * 800.0, 9019.0);
+  const int node = __double2loint(__dadd_rz(__dadd_rz(y, 0.5), 4503599627370496.0));
+  const double2 gw = tab[node];
   double p = fma(c.cZH, gw.y, c.cL2);
   p = fma(L, p, c.bL);
   return fma(L, p, gw.x * c.gG);
@@ -574,53 +588,72 @@ __device__ __forceinline__ double point_xhat64(double chi_c, double T, double nu
   return chi_c + chi_c * Bnu;
 }
 
-// chi_l of a window: NF > 0 in registers; NF = 0 (any window size) in the cell's
-// row of chi_out, which the epilogue then overwrites with the transfer units
-template <int NF>
-struct ChlF64 {
-  double v[NF];
-  __device__ __forceinline__ ChlF64(double *) {}
-  __device__ __forceinline__ double &operator[](int i) { return v[i]; }
-};
-template <>
-struct ChlF64<0> {
-  double *p;
-  __device__ __forceinline__ ChlF64(double *row) : p(row) {}
-  __device__ __forceinline__ double &operator[](int i) { return p[i]; }
-};
+// One line's window into a lane's NF registers of chi_l (LaneWin as in the FP32 kernel)
+template <int NF, bool FULL, bool FAR, bool BIG>
+__device__ __forceinline__ void deposit_window64(double (&chl)[NF], const double2 *tab, const QlgCoef64 &cf, double x0,
+                                                 const LaneWin &w) {
+  const double2 gw = tab[QLG_NTAB - 1];
+  const double p1 = fma(cf.cZH, gw.y, cf.cL2), gg = gw.x * cf.gG;
+#pragma unroll
+  for (int f = 0; f < NF; f++) {
+    const bool hi = f >= NF / 2;
+    if (FULL || (f + 1 >= (hi ? w.ahi : w.alo) && f + 1 <= (hi ? w.bhi : w.blo))) {
+      const double xs = (x0 + ((double)f + (double)(hi ? w.khi : w.klo))) * cf.ih;
+      chl[f] += qlg_eval64<FAR, BIG>(tab, cf, xs, p1, gg);
+    }
+  }
+}
 
-// nray directions share the launch, and with WINS nwin windows (NF > 0), as in
-// k_lte_opacity_units_lane
+// One lane per cell with chi_l of the window in NF double registers, or P lanes a cell
+// for wider windows; nray directions and with WINS nwin windows share the launch, the
+// warps fetching their units, all as in k_lte_opacity_units_lane.  One block of 512
+// threads (128 registers) per SM, the tables in shared memory: 157 registers a thread
+// left one block of 256, an eighth of the warps, and an issue slot in four busy.  The
+// window forms (whole, beyond the table) are chosen by the warp's vote as in FP32, and
+// the reciprocal is two Newton steps unless the window reaches 1 + xs^2 = 1e300: the
+// point costs ten double operations in the usual form, where the general form with its
+// division and table read took some sixty instructions for every line.
 template <int NF, bool WINS = false>
-__global__ void __launch_bounds__(256) k_lte_opacity_units_f64(AtmosDev A, GridArgs G0, const double *nu0,
-                                                               double *chi_out, double *S_out, const double2 *tab,
-                                                               const GridArgs *Gw, int nwin, const double *vr,
-                                                               int nray) {
-  static_assert(!WINS || NF > 0, "window batches of a fixed window size");
+__global__ void __launch_bounds__(512, 1) k_lte_opacity_units_f64(AtmosDev A, GridArgs G0, const double *nu0,
+                                                                  double *chi_out, double *S_out, const double2 *tab,
+                                                                  const GridArgs *Gw, int nwin, const double *vr,
+                                                                  int nray, int P_, int *next) {
+  extern __shared__ __align__(16) double2 s_tab64[];
+  for (int i = threadIdx.x; i < QLG_NTAB; i += blockDim.x) s_tab64[i] = tab[i];
+  __syncthreads();
   const double ex_cutoff = -85.0, voigt_peak = 0.56418958354775628, sqrt_pi = 1.7724538509055160;
   const double tol = (double)G0.tol, flo_scale = (double)G0.flo_scale;
   const double lt = log(tol / voigt_peak);
   const int ncell = A.ncell;
-  const int nf = NF > 0 ? NF : G0.nf;
-  const long long nrc = (long long)nray * ncell;
-  const long long nvc = WINS ? nrc * nwin : nrc;
-  for (long long vc = blockIdx.x * (long long)blockDim.x + threadIdx.x; vc < nvc;
-       vc += (long long)gridDim.x * blockDim.x) {
-    const int w = WINS ? (int)(vc / nrc) : 0;
-    const long long rc = vc - w * nrc;
+  const int nf = WINS ? NF : G0.nf;
+  const int P = WINS ? 1 : P_;
+  const int lane = threadIdx.x & 31;
+  const int sub = lane & (P - 1);
+  const int o = (sub * nf) / P;
+  const int nl = ((sub + 1) * nf) / P - o;
+  const int pad = NF - nl;
+  const unsigned cellmask = P == 32 ? 0xffffffffu : ((1u << P) - 1u) << (lane & ~(P - 1));
+  const int cw = 32 / P;
+  const int upw = (int)(((long long)nray * ncell + cw - 1) / cw);
+  const int nunit = WINS ? upw * nwin : upw;
+  auto fetch = [&]() {
+    int v = 0;
+    if ((threadIdx.x & 31) == 0) v = atomicAdd(next, 1) + gridDim.x * (blockDim.x >> 5);
+    return __shfl_sync(0xffffffffu, v, 0);
+  };
+  for (int u = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; u < nunit; u = fetch()) {
+    const int w = WINS ? u / upw : 0;
+    const long long rc = min((long long)(u - w * upw) * cw + lane / P, (long long)nray * ncell - 1);
     const int ray = (int)(rc / ncell);
     const int cell = (int)(rc - (long long)ray * ncell);
     const GridArgs G = WINS ? Gw[w] : G0;
-    const double *nu = WINS ? nu0 + (size_t)nf * w : nu0;
+    const double *nu = WINS ? nu0 + (size_t)NF * w : nu0;
     const double v0 = vr[3 * ray], v1 = vr[3 * ray + 1], v2 = vr[3 * ray + 2];
     const double sdl = G.inv_dllam;
     const double T = A.temp[cell], chi_c = A.chi_c[cell];
-    const size_t row = WINS ? (size_t)ray * ncell * nwin * nf + (size_t)nf * nwin * cell + (size_t)nf * w
-                            : (size_t)nf * (size_t)rc;
-    double *co = chi_out + row, *so = S_out + row;
-    ChlF64<NF> chl(co);
+    double chl[NF];
 #pragma unroll
-    for (int f = 0; f < nf; f++) chl[f] = 0.0;
+    for (int f = 0; f < NF; f++) chl[f] = 0.0;
     const double vproj = (v0 * (double)A.vx[cell] + v1 * (double)A.vy[cell]) + v2 * (double)A.vz[cell];
     const double ekt = A.e_kT[cell], ne = A.ne[cell], tothi = A.tothi[cell], starkpe = A.stark_pe[cell];
     // xhat and logref at the window edges, where every line centred outside lands
@@ -635,26 +668,24 @@ __global__ void __launch_bounds__(256) k_lte_opacity_units_f64(AtmosDev A, GridA
       const double unsold_c = exp(0.3 * lvb2) * tothi;
       for (int l = 0; l < L.nline; l++) {
         if (L.active && !L.active[l]) continue;
-        const double llc = L.llam0[l] - vproj;
-        const double pos = (llc - G.llam1) * G.inv_dllam;
-        const int ic = (int)lround(pos) + 1;
-        const int f0 = ic < 1 ? 1 : (ic > nf ? nf : ic);
         const double arg = (base + (double)L.gpref[l]) - (double)L.lower_ev[l] * ekt;
         if (arg < ex_cutoff) continue;
+        const double llc = L.llam0[l] - vproj;
+        const double pos = (llc - G.llam1) * G.inv_dllam;
+        const int ic = lround_d(pos) + 1;
+        const int f0 = ic < 1 ? 1 : (ic > nf ? nf : ic);
         double cont0, lr0, chl0;
         if (f0 == 1) { cont0 = x_lo; lr0 = lr_lo; chl0 = chl[0]; }
-        else if (f0 == nf) { cont0 = x_hi; lr0 = lr_hi; chl0 = chl[nf - 1]; }
+        else if (f0 == nf) { cont0 = x_hi; lr0 = lr_hi; chl0 = chl[NF - 1]; }
         else {
           cont0 = point_xhat64(chi_c, T, nu[f0 - 1]);
           lr0 = cont0 > 0.0 ? lt + log(cont0) : -DBL_MAX;
-          if constexpr (NF > 0) {
-            chl0 = chl[0];
+          const int i = f0 - 1 - o, k0 = i >= NF / 2 ? i + pad : i;
+          chl0 = chl[0];
 #pragma unroll
-            for (int k = 1; k < NF; k++) chl0 = (k == f0 - 1) ? chl[k] : chl0;
-          } else {
-            chl0 = chl[f0 - 1];
-          }
+          for (int k = 1; k < NF; k++) chl0 = (k == k0) ? chl[k] : chl0;
         }
+        if (!WINS && P > 1) chl0 = __shfl_sync(cellmask, chl0, (f0 * P - 1) / nf, P);
         double refl = tol * cont0, lref;
         const double flo = flo_scale * chl0;
         if (flo > refl) { refl = flo; lref = log(flo * sqrt_pi); }
@@ -673,28 +704,55 @@ __global__ void __launch_bounds__(256) k_lte_opacity_units_f64(AtmosDev A, GridA
         const double x1 = (G.llam[f0 - 1] - llc) * G.inv_dllam;
         const QlgCoef64 cf = qlg_setup64(a, D, SQ, S);
         const double hw = qlg_halfwidth64(D2, a, S, refl, arg - lref);
-        const int noff = (int)lround(fmin(hw, (double)(nf + abs(ic))));
+        const int noff = lround_d(fmin(hw, (double)(nf + abs(ic))));
         const int fa = ic - noff > 1 ? ic - noff : 1;
         const int fb = ic + noff < nf ? ic + noff : nf;
-        if (fa > fb) continue;
+        const int ga = max(fa, o + 1), gb = min(fb, o + nl);
+        if (ga > gb) continue;
         const double x0 = x1 - (double)(f0 - fa);
-        if constexpr (NF > 0) {
-#pragma unroll
-          for (int f = 0; f < NF; f++)
-            if (f + 1 >= fa && f + 1 <= fb) chl[f] += qlg_eval64(tab, cf, x0 + (double)(f + 1 - fa));
-        } else {
-          for (int f = fa - 1; f < fb; f++) chl[f] += qlg_eval64(tab, cf, x0 + (double)(f + 1 - fa));
-        }
+        LaneWin lw;
+        lw.klo = (float)(o + 1 - fa);
+        lw.khi = (float)(o - pad + 1 - fa);
+        lw.alo = fa - o;
+        lw.blo = fb - o;
+        lw.ahi = lw.alo + pad;
+        lw.bhi = lw.blo + pad;
+        const double xb = x0 + (double)(ga - fa), xe = x0 + (double)(gb - fa);
+        const double xnear = xb > 0.0 ? xb : (xe < 0.0 ? -xe : 0.0);
+        const unsigned conv = __activemask();
+        const bool full = __all_sync(conv, fa <= o + 1 && fb >= o + nl);
+        const bool far = __all_sync(conv, fmin(xnear * cf.ih * 800.0, 9019.0) >= 9018.5);
+        if (!__all_sync(conv, fmax(fabs(xb), fabs(xe)) * cf.ih <= 1e150))
+          deposit_window64<NF, false, false, true>(chl, s_tab64, cf, x0, lw);
+        else if (far && full)
+          deposit_window64<NF, true, true, false>(chl, s_tab64, cf, x0, lw);
+        else if (full)
+          deposit_window64<NF, true, false, false>(chl, s_tab64, cf, x0, lw);
+        else
+          deposit_window64<NF, false, false, false>(chl, s_tab64, cf, x0, lw);
       }
     }
-    // epilogue: transfer units (in place over the accumulator row when NF = 0)
-#pragma unroll
-    for (int f = 0; f < nf; f++) {
-      double c, sv;
-      point_units(chi_c, T, nu[f], chl[f], chl[f], (double)A.maser_chi_floor, c, sv);
-      co[f] = c;
-      so[f] = sv;
+    // epilogue: transfer units; the frequencies both register halves hold are written
+    // once, from the first
+    size_t row;
+    {
+      int ue = u;
+      asm volatile("" : "+r"(ue));
+      const int we = WINS ? ue / upw : 0;
+      const long long re = (long long)(ue - we * upw) * cw + (threadIdx.x & 31) / P;
+      if (re >= (long long)nray * ncell) continue;
+      row = WINS ? (size_t)NF * nwin * (size_t)re + (size_t)NF * we : (size_t)nf * (size_t)re;
     }
+    double *co = chi_out + row, *so = S_out + row;
+#pragma unroll
+    for (int k = 0; k < NF; k++)
+      if (k < NF / 2 || k - pad >= NF / 2) {
+        const int f = o + (k < NF / 2 ? k : k - pad);
+        double c, sv;
+        point_units(chi_c, T, nu[f], chl[k], chl[k], (double)A.maser_chi_floor, c, sv);
+        co[f] = c;
+        so[f] = sv;
+      }
   }
 }
 

@@ -41,3 +41,16 @@ def test_rays_together_equal_one_by_one(m3d, nf, fp64):
     for r in (0, 4, 12):
         ie1, _, top1 = m3d.lte_synthesis(atm, nu, llam, vec[r:r + 1], wmu[r:r + 1], fp64=fp64, return_itop=True)
         assert np.array_equal(top[r], top1[0]) and np.array_equal(ie[r], ie1[0])
+
+
+@pytest.mark.parametrize("nf", [2, 3, 5, 8, 9, 16, 17, 31, 33, 64, 65, 100, 257])
+def test_double_window_sizes(m3d, oracle, nf):
+    """The plain FP64 pass at the edges of its register counts (4, 8, 16, 32 frequencies
+    a lane, then several lanes a cell), to 1e-11: the device's double exp and log."""
+    from oracle import pipeline as P
+    atm, nu, llam, vec, _ = _case(nf, 3)
+    for v in vec[:1] if nf > 64 else vec:
+        chi, S = m3d.lte_transfer_units(atm, nu, llam, v, fp64=True)
+        ochi, oS = P.transfer_units(atm, nu, llam, v, fp64=True)
+        np.testing.assert_allclose(chi, ochi, rtol=1e-11, atol=0)
+        np.testing.assert_allclose(S, oS, rtol=1e-11, atol=0)
