@@ -811,38 +811,70 @@ int solve_impl(int solver, const m3d_slab_t *s, unsigned flags, T *work, T *psi,
                       "the stencil reaches one cell (ds_x >= |v_x/v_z| ds_z)",
                       s->vec[0], s->vec[1], s->vec[2], wt1, wt2);
       }
-      std::vector<int> tab(4 * (a.nx + a.ny));
-      for (int x = 0; x < a.nx; x++)
-        for (int ii = 0; ii < 4; ii++) {
-          int v = ((ii + 1) + (x + 1) + (upo1 - 2)) % a.nx;
-          tab[4 * x + ii] = v < 0 ? v + a.nx : v;
-        }
-      for (int y = 0; y < a.ny; y++)
-        for (int jj = 0; jj < 4; jj++) {
-          int v = ((jj + 1) + (y + 1) + (upo2 - 2)) % a.ny;
-          tab[4 * a.nx + 4 * y + jj] = v < 0 ? v + a.ny : v;
-        }
-      void *dtab;
-      TRY(scratch(3, sizeof(int) * tab.size(), &dtab));
-      CUDA_TRY(cudaMemcpyAsync(dtab, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice, g_ctx.stream));
-      const int *xt = (const int *)dtab, *yt = xt + 4 * a.nx;
       const float4 kx = make_float4((float)xk[0], (float)xk[1], (float)xk[2], (float)xk[3]);
       const float4 ky = make_float4((float)yk[0], (float)yk[1], (float)yk[2], (float)yk[3]);
       const int zs = a.dir > 0 ? 1 : a.nz;
       if (solver == M3D_SOLVER_SHORT_LINEAR) {
         const T dsup05 = (T)(0.5f * (float)dsup);
         const size_t smem = sizeof(T) * 3 * (SC_TX + 3) * (SC_TY + 3) * SC_TF;
-        thread_local bool attr_set[2] = {false, false};
-        if (!attr_set[sizeof(T) == 8]) {
-          CUDA_TRY(cudaFuncSetAttribute(k_short_char_tile<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-          attr_set[sizeof(T) == 8] = true;
-        }
+        // elements a staging copy: every row of frequencies starts on a multiple of them
+        const int elems = (int)(16 / sizeof(T));
+        int vec = 1;
+        while (2 * vec <= elems && a.nf % (2 * vec) == 0 && (uintptr_t)work % (2 * vec * sizeof(T)) == 0) vec *= 2;
+        using TileKernel = void (*)(SlabArgs, int, T *, T *, T *, T *, int, int, float4, float4, T);
+        TileKernel kern = vec == 1 ? (TileKernel)k_short_char_tile<T, 1> : (TileKernel)k_short_char_tile<T, 2>;
+        if constexpr (sizeof(T) == 4)
+          if (vec == 4) kern = k_short_char_tile<T, 4>;
+        CUDA_TRY(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         const int tgrid = ((a.nx + SC_TX - 1) / SC_TX) * ((a.ny + SC_TY - 1) / SC_TY) * ((a.nf + SC_TF - 1) / SC_TF);
-        for (int i = 0, z = zs; i < a.nz; i++, z += a.dir)
-          LAUNCH_S(M3D_STAGE_SOLVE, k_short_char_tile<T>, tgrid, 256, smem, a, z, work, psi, irem, esc, xt, yt, kx, ky,
-                   dsup05);
+        const int x1 = wrap_host(upo1, a.nx), y1 = wrap_host(upo2, a.ny);
+        for (int i = 0, z = zs; i < a.nz; i++, z += a.dir) {
+          if (i == 0) {
+            LAUNCH_S(M3D_STAGE_SOLVE, kern, tgrid, 256, smem, a, z, work, psi, irem, esc, x1, y1, kx, ky, dsup05);
+            continue;
+          }
+          // the next plane behind this one, its start overlapping this one's end
+          cudaLaunchAttribute at;
+          at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+          at.val.programmaticStreamSerializationAllowed = 1;
+          cudaLaunchConfig_t cfg = {};
+          cfg.gridDim = dim3(tgrid);
+          cfg.blockDim = dim3(256);
+          cfg.dynamicSmemBytes = smem;
+          cfg.stream = g_ctx.stream;
+          cfg.attrs = &at;
+          cfg.numAttrs = 1;
+          cudaEvent_t ea = nullptr, eb = nullptr;
+          if (g_ctx.profile) {
+            ea = take_event();
+            eb = take_event();
+            cudaEventRecord(ea, g_ctx.stream);
+          }
+          CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a, z, work, psi, irem, esc, x1, y1, kx, ky, dsup05));
+          g_ctx.launches++;
+          if (g_ctx.profile) {
+            cudaEventRecord(eb, g_ctx.stream);
+            g_ctx.recs.push_back(Ctx::Rec{M3D_STAGE_SOLVE, ea, eb});
+          }
+        }
+        return M3D_OK;
       } else {
         if (!chi500 || !chi500_up || !g500) return fail(M3D_EINVAL, "linear2 needs chi500, chi500_up and g500");
+        std::vector<int> tab(4 * (a.nx + a.ny));
+        for (int x = 0; x < a.nx; x++)
+          for (int ii = 0; ii < 4; ii++) {
+            int v = ((ii + 1) + (x + 1) + (upo1 - 2)) % a.nx;
+            tab[4 * x + ii] = v < 0 ? v + a.nx : v;
+          }
+        for (int y = 0; y < a.ny; y++)
+          for (int jj = 0; jj < 4; jj++) {
+            int v = ((jj + 1) + (y + 1) + (upo2 - 2)) % a.ny;
+            tab[4 * a.nx + 4 * y + jj] = v < 0 ? v + a.ny : v;
+          }
+        void *dtab;
+        TRY(scratch(3, sizeof(int) * tab.size(), &dtab));
+        CUDA_TRY(cudaMemcpyAsync(dtab, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice, g_ctx.stream));
+        const int *xt = (const int *)dtab, *yt = xt + 4 * a.nx;
         const float hx = 2.0f * kx.w + (-kx.x + kx.z), hy = 2.0f * ky.w + (-ky.x + ky.z);
         for (int i = 0, z = zs; i < a.nz; i++, z += a.dir)
           LAUNCH_S(M3D_STAGE_SOLVE, k_short_char2_plane<T>, grid, block, 0, a, z, work, psi, irem, esc, xt, yt, kx, ky, hx, hy, chi500,

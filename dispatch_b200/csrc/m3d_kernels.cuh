@@ -977,19 +977,31 @@ __global__ void k_upstream_boundary(int nf, int nx, int ny, int nz, int dir, T *
 // consecutive upstream columns starting at xt[4 x0].
 constexpr int SC_TX = 8, SC_TY = 8, SC_TF = 32;
 
-// one element global -> shared without a register round trip (cp.async, sm_80+);
-// all of a block's copies are in flight together and complete at cp_async_wait_all
-template <typename T>
-__device__ __forceinline__ void cp_async_elem(T *dst, const T *src) {
+// BYTES (4, 8 or 16, both addresses aligned to them) global -> shared without a register
+// round trip (cp.async); all of a block's copies are in flight together and complete at
+// cp_async_wait_all
+template <int BYTES>
+__device__ __forceinline__ void cp_async_bytes(void *dst, const void *src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(src), "n"(sizeof(T)));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(src), "n"(BYTES));
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-template <typename T>
+// Programmatic dependent launch: wait for the grid this one was launched behind (at once
+// for a plain launch), and let the next one's blocks start as room appears.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// VEC elements a copy: 16, 8 or 4 bytes as nf and work's alignment allow (one element a
+// copy, with a row's place divided out for each, the staging was a third of the
+// kernel's instructions).  x1, y1: the upstream column and row of the first stencil,
+// xt[0] and yt[0].  The planes are launched as a chain of dependent grids: a plane
+// stages the upstream chi and S and loads its own, which no plane writes, while the plane
+// before it ends, and waits for that one before it reads its intensities.  48^3 cells and
+// 250 frequencies, a plane: 18.9 -> 9.9 us by the kernel, 26 directions 22.1 -> 12.4 ms.
+template <typename T, int VEC>
 __global__ void __launch_bounds__(256) k_short_char_tile(SlabArgs s, int z, T *work, T *psi, T *irem, T *esc,
-                                                         const int *xt, const int *yt, float4 kx, float4 ky,
-                                                         T dsup05) {
+                                                         int x1, int y1, float4 kx, float4 ky, T dsup05) {
   extern __shared__ __align__(16) unsigned char sc_smem[];
   T *up = (T *)sc_smem;  // [3][SC_TY+3][SC_TX+3][SC_TF]
   constexpr int PX = SC_TX + 3, PY = SC_TY + 3;
@@ -1000,32 +1012,49 @@ __global__ void __launch_bounds__(256) k_short_char_tile(SlabArgs s, int z, T *w
   const int tx = bt % ntx, ty = (bt / ntx) % nty, fc = bt / (ntx * nty);
   const int x0 = tx * SC_TX, y0 = ty * SC_TY, f0 = fc * SC_TF;
   const int zup = z - dir;
-  if (threadIdx.x < PX) sxu[threadIdx.x] = (xt[4 * x0] + threadIdx.x) % nx;
-  else if (threadIdx.x < PX + PY) syu[threadIdx.x - PX] = (yt[4 * y0] + threadIdx.x - PX) % ny;
+  if (threadIdx.x < PX) sxu[threadIdx.x] = (x1 + x0 + threadIdx.x) % nx;
+  else if (threadIdx.x < PX + PY) syu[threadIdx.x - PX] = (y1 + y0 + threadIdx.x - PX) % ny;
   __syncthreads();
-  // one warp per upstream row of SC_TF frequencies (coalesced)
-  {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const bool fin = f0 + lane < nf && lane < SC_TF;
-    const size_t plane = (size_t)nf * nx * ny, slot = plane * (nz + 2);
-    for (int row = wid; row < 3 * PY * PX; row += nw) {
-      const int xi = row % PX, yj = (row / PX) % PY, i = row / (PX * PY);
-      const size_t base = slot * i + plane * zup + (size_t)nf * (sxu[xi] + (size_t)nx * syu[yj]) + f0;
-      if (fin) cp_async_elem(&up[row * SC_TF + lane], &work[base + lane]);
+  // a warp per upstream row of columns, VEC columns of SC_TF frequencies at a time
+  const size_t plane = (size_t)nf * nx * ny, k1 = plane * (nz + 2);
+  auto stage = [&](int i0, int i1) {
+    const int sub = (threadIdx.x & 31) / (32 / VEC), fl = (threadIdx.x & 31) % (32 / VEC) * VEC;
+    if (f0 + fl >= nf) return;
+    for (int p = i0 * PY + (threadIdx.x >> 5); p < i1 * PY; p += 8) {
+      const int i = p / PY, yj = p - i * PY;
+      const T *src = work + k1 * i + plane * zup + (size_t)nf * ((size_t)nx * syu[yj]) + (f0 + fl);
+      T *dst = up + (size_t)p * PX * SC_TF + fl;
+      for (int xi = sub; xi < PX; xi += VEC)
+        cp_async_bytes<VEC * (int)sizeof(T)>(dst + xi * SC_TF, src + (size_t)nf * sxu[xi]);
     }
-    cp_async_wait_all();
-  }
-  __syncthreads();
-  const T dtmax = -(T)s.maser_dtau_max, Imax = (T)s.maser_Inu_max;
-  const T k_x[4] = {(T)kx.x, (T)kx.y, (T)kx.z, (T)kx.w};
-  const T k_y[4] = {(T)ky.x, (T)ky.y, (T)ky.z, (T)ky.w};
+  };
+  stage(0, 2);
   // one warp per column x of the tile, lanes along f, sliding down y: the row sums
   // of an upstream row serve the four targets whose stencils hold it
   const int lane = threadIdx.x & 31, xl = threadIdx.x >> 5;
   const int x = x0 + xl, f = lane;
-  if (x >= nx || f0 + f >= nf || xl >= SC_TX) return;
-  const size_t plane = (size_t)nf * nx * ny, k1 = plane * (nz + 2);
+  const bool mine = x < nx && f0 + f < nf;
   const size_t pz = plane * (size_t)z, pp = plane * (size_t)(z - 1);
+  // this column's chi and S on plane z for all the tile's rows, loaded up front
+  T xxv[SC_TY], ssv[SC_TY];
+  if (mine) {
+#pragma unroll
+    for (int yl = 0; yl < SC_TY; yl++) {
+      const int y = y0 + yl < ny ? y0 + yl : ny - 1;
+      const size_t o = pz + (size_t)nf * ((size_t)x + (size_t)nx * (size_t)y) + (size_t)(f0 + f);
+      xxv[yl] = work[o];
+      ssv[yl] = work[o + k1];
+    }
+  }
+  grid_dependency_wait();
+  grid_dependents_launch();
+  stage(2, 3);
+  cp_async_wait_all();
+  __syncthreads();
+  if (!mine) return;
+  const T dtmax = -(T)s.maser_dtau_max, Imax = (T)s.maser_Inu_max;
+  const T k_x[4] = {(T)kx.x, (T)kx.y, (T)kx.z, (T)kx.w};
+  const T k_y[4] = {(T)ky.x, (T)ky.y, (T)ky.z, (T)ky.w};
   constexpr int RS = PX * SC_TF;   // one upstream row in shared memory
   constexpr int FS = PY * RS;      // one field
   const T *u0 = up + (size_t)xl * SC_TF + f;
@@ -1043,15 +1072,6 @@ __global__ void __launch_bounds__(256) k_short_char_tile(SlabArgs s, int z, T *w
       v2[i][slot] = row[2 * SC_TF];
     }
   };
-  // this column's chi and S on plane z for all the tile's rows, loaded up front
-  T xxv[SC_TY], ssv[SC_TY];
-#pragma unroll
-  for (int yl = 0; yl < SC_TY; yl++) {
-    const int y = y0 + yl < ny ? y0 + yl : ny - 1;
-    const size_t o = pz + (size_t)nf * ((size_t)x + (size_t)nx * (size_t)y) + (size_t)(f0 + f);
-    xxv[yl] = work[o];
-    ssv[yl] = work[o + k1];
-  }
 #pragma unroll
   for (int jj = 0; jj < 3; jj++) load_row(jj, jj);
 #pragma unroll
