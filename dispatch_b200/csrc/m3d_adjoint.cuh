@@ -181,14 +181,24 @@ __device__ __forceinline__ void rot_at(const float *chi, const float *S, size_t 
 // Outputs dL/d(rotated chi) and dL/d(rotated S) of every plane in g_xrot/g_srot
 // ((nf, nx, ny, nz), the sweep's own frame), and the PCHIP ghost's partials in the
 // bottom two unrotated planes in g_ghost (4, nf, nx, ny): chi(1), chi(2), S(1), S(2).
+// The rays of a group run along grid.y, every array ray after ray.
 __global__ void __launch_bounds__(128) k_quad_rot_column_adj(int nf, int nx, int ny, int nz, const float *chi,
                                                              const float *S, const RotCol *rot, const int *slab_z0,
-                                                             int nslab, QuadConst qc, PchipConst pc, float dtmax,
-                                                             float Imax, const float *g_top, float *g_xrot,
-                                                             float *g_srot, float *g_ghost) {
+                                                             int nslab, const QuadConst *qcs, PchipConst pc,
+                                                             float dtmax, float Imax, const float *g_top,
+                                                             float *g_xrot, float *g_srot, float *g_ghost) {
   const size_t plane = (size_t)nf * nx * ny;
   const size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (g >= plane) return;
+  const QuadConst qc = qcs[blockIdx.y];
+  const size_t column = plane * nz * blockIdx.y;
+  chi += column;
+  S += column;
+  rot += (size_t)nz * blockIdx.y;
+  g_top += plane * blockIdx.y;
+  g_xrot += column;
+  g_srot += column;
+  g_ghost += 4 * plane * blockIdx.y;
   const int f = (int)(g % nf), x = (int)((g / nf) % nx), y = (int)(g / ((size_t)nf * nx));
   // ghost
   float d_c1, d_c2, d_s1, d_s2;
@@ -283,11 +293,18 @@ __global__ void __launch_bounds__(128) k_quad_rot_column_adj(int nf, int nx, int
 __global__ void k_unrotate_adj(int nf, int nx, int ny, int nz, const RotCol *rot, const float *g_xrot,
                                const float *g_srot, const float *g_ghost, float *g_chi, float *g_S) {
   const size_t plane = (size_t)nf * nx * ny;
-  const size_t n = plane * nz;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
-    const size_t in = t % plane;
-    const int z = (int)(t / plane);
-    const int f = (int)(in % nf), x = (int)((in / nf) % nx), y = (int)(in / ((size_t)nf * nx));
+  const size_t in = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (in >= plane) return;
+  const int f = (int)(in % nf), x = (int)((in / nf) % nx), y = (int)(in / ((size_t)nf * nx));
+  const size_t column = plane * nz * blockIdx.y;       // rays along grid.y
+  g_xrot += column;
+  g_srot += column;
+  g_ghost += 4 * plane * blockIdx.y;
+  g_chi += column;
+  g_S += column;
+  rot += (size_t)nz * blockIdx.y;
+  for (int z = blockIdx.z; z < nz; z += gridDim.z) {
+    const size_t t = in + plane * z;
     const RotCol r = rot[z];
     int xa = x - r.ux; xa = xa < 0 ? xa + nx : xa;          // columns whose first tap is x
     int xb = xa - 1; xb = xb < 0 ? xb + nx : xb;            // whose second tap is x
@@ -308,14 +325,16 @@ __global__ void k_unrotate_adj(int nf, int nx, int ny, int nz, const RotCol *rot
 
 // The transfer units of every point from its line opacity chi_l (the opacity
 // kernel's epilogue on its own): chil, chi, S (nf, ncell)
-__global__ void k_units_fwd(int nf, int ncell, const double *nu, const float *temp, const float *chi_c,
+// windows of 32 frequencies, rays along grid.y
+__global__ void k_units_fwd(int ncell, const double *nu, const float *temp, const float *chi_c,
                             float maser_chi_floor, const float *chil, float *chi, float *S) {
-  const size_t n = (size_t)nf * ncell;
+  const size_t n = (size_t)32 * ncell, ray = n * blockIdx.y;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i / nf), f = (int)(i % nf);
+    const int c = (int)(i >> 5), f = (int)(i & 31);
     const float T = temp[c];
     const float h_kT = (float)(M3D_H_K / (double)T);
-    point_units(chi_c[c], h_kT, nu[f], chil[i], chil[i], maser_chi_floor, chi[i], S[i]);
+    const float cl = chil[ray + i];
+    point_units(chi_c[c], h_kT, nu[f], cl, cl, maser_chi_floor, chi[ray + i], S[ray + i]);
   }
 }
 
@@ -362,21 +381,38 @@ __device__ __forceinline__ float units_adj(float chi_c, float T, float h_kT, dou
   return g_w1 + g_w2;
 }
 
-// k_units_adj: one thread per cell, its window's frequencies in order.  chil, g_chi,
-// g_S: (nf, ncell); writes g_chil and adds into g_temp and g_chic.
-__global__ void k_units_adj(int nf, int ncell, const double *nu, const float *temp, const float *chi_c,
+// k_units_adj: a warp per cell, lanes along the window's 32 frequencies (a thread per cell
+// read rows 128 bytes apart: 95 us a ray of 65536 cells), rays along grid.y.  chil, g_chi,
+// g_S: (nf, ncell) per ray; writes g_chil and the ray's dL/dT and dL/dchi_c of the cell.
+__global__ void k_units_adj(int ncell, const double *nu, const float *temp, const float *chi_c,
                             float maser_chi_floor, const float *chil, const float *g_chi, const float *g_S,
-                            float *g_chil, float *g_temp, float *g_chic) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x) {
-    const float T = temp[c], cc = chi_c[c];
+                            float *g_chil, float *p_temp, float *p_chic) {
+  const size_t n = (size_t)32 * ncell, ray = n * blockIdx.y;
+  // whole warps: n and the stride are multiples of 32
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const int c = (int)(i >> 5), f = (int)(i & 31);
+    const float T = temp[c];
     const float h_kT = (float)(M3D_H_K / (double)T);
     float gT = 0.0f, gC = 0.0f;
-    for (int f = 0; f < nf; f++) {
-      const size_t i = (size_t)f + (size_t)nf * c;
-      g_chil[i] = units_adj(cc, T, h_kT, nu[f], chil[i], maser_chi_floor, g_chi[i], g_S[i], gT, gC);
+    g_chil[ray + i] = units_adj(chi_c[c], T, h_kT, nu[f], chil[ray + i], maser_chi_floor, g_chi[ray + i],
+                                g_S[ray + i], gT, gC);
+    for (int o = 16; o > 0; o >>= 1) {
+      gT += __shfl_xor_sync(0xffffffffu, gT, o);
+      gC += __shfl_xor_sync(0xffffffffu, gC, o);
     }
-    g_temp[c] += gT;
-    g_chic[c] += gC;
+    if (f == 0) {
+      p_temp[(size_t)ncell * blockIdx.y + c] = gT;
+      p_chic[(size_t)ncell * blockIdx.y + c] = gC;
+    }
+  }
+}
+
+// g += the rays' parts, in the rays' order
+__global__ void k_add_rays(size_t n, int nray, const float *part, float *g) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    float v = g[i];
+    for (int r = 0; r < nray; r++) v += part[n * r + i];
+    g[i] = v;
   }
 }
 
@@ -426,59 +462,119 @@ __device__ __forceinline__ float qlg_eval_d(const float2 *tab, const float *dW, 
 
 // One line's window replayed: chl gets the forward's K bit for bit (the forms the
 // forward chooses by warp vote all give the general form's bits), Gl and Hl the sums
-// of g_chil K and g_chil dK/dih.  FAR: every point beyond the table, whose last node
-// gives G, W and W' at every point, so the per-point work is the forward's far form
-// plus the derivative's few terms.
-template <int NF, bool FULL, bool FAR, bool MK>
+// of g_chil K and g_chil dK/dih.  This is the general form, point by point.
+template <int NF>
 __device__ __forceinline__ void deposit_adj(float (&chl)[NF], const float (&gch)[NF], const float2 *s_tab,
                                             const float *s_dW, const QlgCoef &cf, const QlgCoefD &cd, float x0,
                                             float kfa, int fa, int fb, float &Gl, float &Hl) {
-  if (FAR) {
-    const float2 gw = s_tab[QLG_NTAB - 1];
-    const float p1 = fmaf(cf.cZH, gw.y, cf.cL2);
-    const float gg = gw.x * cf.gG;
-    const float ca = cf.cZH * s_dW[QLG_NTAB - 1], cb = -0.69314718f * gg;
-    const float e1 = fmaf(gw.y, cd.cZH, cd.cL2), e3 = gw.x * cd.gG;
-    const float r2ih = 2.0f / cf.ih;
 #pragma unroll
-    for (int f = 0; f < NF; f++) {
-      if (FULL || (f + 1 >= fa && f + 1 <= fb)) {
-        const float xs = fabsf(x0 + (FULL ? (float)f : ((float)f + kfa))) * cf.ih;
-        const float u = xs * xs;
-        const float L = qlg_rcp<MK>(1.0f + u);
-        const float K = fmaf(L, fmaf(L, p1, cf.bL), gg);
-        chl[f] = fmaf(K, 1.0f, chl[f]);
-        const float dK_du = fmaf(L * L, ca - fmaf(2.0f * L, p1, cf.bL), cb);
-        const float dKi = fmaf(dK_du, u * r2ih, fmaf(L, fmaf(L, e1, cd.bL), e3));
-        Gl = fmaf(gch[f], K, Gl);
-        Hl = fmaf(gch[f], dKi, Hl);
-      }
-    }
-  } else {
-#pragma unroll
-    for (int f = 0; f < NF; f++) {
-      if (FULL || (f + 1 >= fa && f + 1 <= fb)) {
-        float dKi;
-        const float K = qlg_eval_d<MK>(s_tab, s_dW, cf, cd, x0 + (FULL ? (float)f : ((float)f + kfa)), dKi);
-        chl[f] = fmaf(K, 1.0f, chl[f]);
-        Gl = fmaf(gch[f], K, Gl);
-        Hl = fmaf(gch[f], dKi, Hl);
-      }
+  for (int f = 0; f < NF; f++) {
+    if (f + 1 >= fa && f + 1 <= fb) {
+      float dKi;
+      const float K = qlg_eval_d<false>(s_tab, s_dW, cf, cd, x0 + ((float)f + kfa), dKi);
+      chl[f] = fmaf(K, 1.0f, chl[f]);
+      Gl = fmaf(gch[f], K, Gl);
+      Hl = fmaf(gch[f], dKi, Hl);
     }
   }
 }
 
-template <int NF, bool MK>
-__device__ __forceinline__ void deposit_adj_mk(float (&chl)[NF], const float (&gch)[NF], const float2 *s_tab,
+// The same, two points per instruction, where every 1 + xs^2 is below 2^126: K as
+// deposit_window_x2 forms it, and dK/dih by
+//   dK/du = L^2 (cZH W' - (2 L P + bL)) - ln2 G gG,  P = cZH W + cL2,
+//   dK/dih = dK/du 2 u/ih + L (L (W dcZH + dcL2) + dbL) + G dgG,
+// FAR: W, W' and G the last node's at every point.  Points outside a partial window add
+// K = 0 and have their sensitivity left out.  The scalar form took some 24 instructions
+// a point, this one 13.
+template <int NF, bool FULL, bool FAR>
+__device__ __forceinline__ void deposit_adj_x2(float (&chl)[NF], const float (&gch)[NF], const float2 *s_tab,
                                                const float *s_dW, const QlgCoef &cf, const QlgCoefD &cd, float x0,
-                                               float kfa, int fa, int fb, bool full, bool far, float &Gl, float &Hl) {
-  if (far) {
-    if (full) deposit_adj<NF, true, true, MK>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
-    else deposit_adj<NF, false, true, MK>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
+                                               float kfa, int fa, int fb, float &Gl, float &Hl) {
+  const f32x2 X0 = splat2(x0), IH = splat2(cf.ih), ONE = splat2(1.0f), NEG = splat2(-1.0f), BL = splat2(cf.bL);
+  const f32x2 KF = splat2(kfa), R2IH = splat2(2.0f / cf.ih), DBL = splat2(cd.bL);
+  f32x2 P1 = 0, GG = 0, CA = 0, CB = 0, E1 = 0, E3 = 0, CZH = 0, CL2 = 0, GGc = 0, DZ = 0, DL = 0, DG = 0, NLN = 0;
+  unsigned base = 0;
+  if (FAR) {
+    const float2 gw = s_tab[QLG_NTAB - 1];
+    const float gg = gw.x * cf.gG;
+    P1 = splat2(fmaf(cf.cZH, gw.y, cf.cL2));
+    GG = splat2(gg);
+    CA = splat2(cf.cZH * s_dW[QLG_NTAB - 1]);
+    CB = splat2(-0.69314718f * gg);
+    E1 = splat2(fmaf(gw.y, cd.cZH, cd.cL2));
+    E3 = splat2(gw.x * cd.gG);
   } else {
-    if (full) deposit_adj<NF, true, false, MK>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
-    else deposit_adj<NF, false, false, MK>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
+    CZH = splat2(cf.cZH);
+    CL2 = splat2(cf.cL2);
+    GGc = splat2(cf.gG);
+    DZ = splat2(cd.cZH);
+    DL = splat2(cd.cL2);
+    DG = splat2(cd.gG);
+    NLN = splat2(-0.69314718f);
+    base = (unsigned)__cvta_generic_to_shared(s_tab) - (0x4B000000u << 3);
   }
+  f32x2 G2 = splat2(0.0f), H2 = splat2(0.0f);
+#pragma unroll
+  for (int k = 0; k < NF / 2; k++) {
+    f32x2 F = pk2((float)(2 * k), (float)(2 * k + 1));
+    if (!FULL) F = add2(F, KF);
+    const f32x2 xs = mul2(add2(X0, F), IH);
+    float xa, xb;
+    up2(xs, xa, xb);
+    const float ua = xa * xa, ub = xb * xb;
+    const float da = 1.0f + ua, db = 1.0f + ub;
+    const f32x2 nd = pk2(-da, -db);
+    const f32x2 r = pk2(rcp_approx(da), rcp_approx(db));
+    const f32x2 L = fma2(r, fma2(nd, r, ONE), r);
+    f32x2 P, gG, cWd, e, eg;
+    f32x2 K;
+    if (FAR) {
+      P = P1;
+      K = fma2(L, fma2(L, P1, BL), GG);
+      gG = CB;
+      cWd = CA;
+      e = E1;
+      eg = E3;
+    } else {
+      const f32x2 y = pk2(fminf(fabsf(xa) * 800.0f, 9019.0f), fminf(fabsf(xb) * 800.0f, 9019.0f));
+      const f32x2 v = add2_rz(add2_rz(y, splat2(0.5f)), splat2(8388608.0f));
+      float va, vb;
+      up2(v, va, vb);
+      const unsigned ia = __float_as_uint(va), ib = __float_as_uint(vb);
+      const float2 ga = lds_node(base + (ia << 3)), gb = lds_node(base + (ib << 3));
+      const f32x2 W = pk2(ga.y, gb.y), G = pk2(ga.x, gb.x);
+      P = fma2(CZH, W, CL2);
+      const f32x2 gg = mul2(G, GGc);
+      K = fma2(L, fma2(L, P, BL), gg);
+      gG = mul2(NLN, gg);
+      cWd = mul2(CZH, pk2(s_dW[ia - 0x4B000000u], s_dW[ib - 0x4B000000u]));
+      e = fma2(W, DZ, DL);
+      eg = mul2(G, DG);
+    }
+    const f32x2 t = fma2(NEG, fma2(add2(L, L), P, BL), cWd);
+    const f32x2 dKu = fma2(mul2(L, L), t, gG);
+    f32x2 dKi = fma2(dKu, mul2(pk2(ua, ub), R2IH), fma2(L, fma2(L, e, DBL), eg));
+    if (!FULL) {
+      float ka, kb, ha, hb;
+      up2(K, ka, kb);
+      up2(dKi, ha, hb);
+      const bool ina = 2 * k + 1 >= fa && 2 * k + 1 <= fb, inb = 2 * k + 2 >= fa && 2 * k + 2 <= fb;
+      K = pk2(ina ? ka : 0.0f, inb ? kb : 0.0f);
+      dKi = pk2(ina ? ha : 0.0f, inb ? hb : 0.0f);
+    }
+    float lo, hi;
+    up2(add2(K, pk2(chl[2 * k], chl[2 * k + 1])), lo, hi);
+    chl[2 * k] = lo;
+    chl[2 * k + 1] = hi;
+    const f32x2 gc = pk2(gch[2 * k], gch[2 * k + 1]);
+    G2 = fma2(gc, K, G2);
+    H2 = fma2(gc, dKi, H2);
+  }
+  float lo, hi;
+  up2(G2, lo, hi);
+  Gl += lo + hi;
+  up2(H2, lo, hi);
+  Hl += lo + hi;
 }
 
 // k_opacity_adj: the line loop of k_lte_opacity_units_lane<32> (no select_lines
@@ -486,13 +582,17 @@ __device__ __forceinline__ void deposit_adj_mk(float (&chl)[NF], const float (&g
 // deposited point adding g_chil(f) K and g_chil(f) dK/dD.  Per depositing line: the
 // sums go to dL/dlnbase (K is proportional to exp(arg)), dL/de_kT (-lower_ev times
 // it), dL/dinv_df (through D = sdl/idf, in S = Rij D and the profile's width) and,
-// reduced over the warp's cells and then the block, dL/dgpref of the line.
+// reduced over the warp's cells and then the block, dL/dgpref of the line.  nray rays
+// share the launch, the warps fetching their units as in the forward kernel; a ray's
+// per-cell sums go to its own part (p_*, ray after ray), which k_add_rays adds in the
+// rays' order, so that these gradients do not depend on the launch.
 // Shared memory: the QLG tables (float2), the table differences dW, and the block's
 // per-line sums (nline floats).
-__global__ void __launch_bounds__(512, 1) k_opacity_adj(AtmosDev A, GridArgs G, const double *nu, double v0,
-                                                        double v1, double v2, const float2 *tab, const float *dWg,
-                                                        const float *g_chil, float *g_lnbase, float *g_ekt,
-                                                        float *g_idf, float *const *g_gpref, int nline_max) {
+__global__ void __launch_bounds__(512, 1) k_opacity_adj(AtmosDev A, GridArgs G, const double *nu, const double *vr,
+                                                        int nray, const float2 *tab, const float *dWg,
+                                                        const float *g_chil, float *p_lnbase, float *p_ekt,
+                                                        float *p_idf, float *const *g_gpref, int nline_max,
+                                                        int *next) {
   namespace cg = cooperative_groups;
   constexpr int NF = 32;
   extern __shared__ float smem[];
@@ -508,18 +608,26 @@ __global__ void __launch_bounds__(512, 1) k_opacity_adj(AtmosDev A, GridArgs G, 
   const float ex_cutoff = -85.0f, voigt_peak = 0.5641895835f, sqrt_pi = 1.7724538509f;
   const float lt = logf_m3d(G.tol / voigt_peak);
   const int ncell = A.ncell;
-  const int ncell_pad = (ncell + 31) / 32 * 32;
   const double llam_hi = G.llam[NF - 1];
-  for (int cell = blockIdx.x * blockDim.x + threadIdx.x; cell < ncell_pad; cell += gridDim.x * blockDim.x) {
-    const bool live = cell < ncell;
-    const int cs = live ? cell : ncell - 1;
+  const int nunit = (int)(((long long)nray * ncell + 31) / 32);
+  auto fetch = [&]() {
+    int v = 0;
+    if ((threadIdx.x & 31) == 0) v = atomicAdd(next, 1) + gridDim.x * (blockDim.x >> 5);
+    return __shfl_sync(0xffffffffu, v, 0);
+  };
+  for (int unit = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; unit < nunit; unit = fetch()) {
+    const long long rc0 = (long long)unit * 32 + (threadIdx.x & 31);
+    const bool live = rc0 < (long long)nray * ncell;
+    const long long rc = live ? rc0 : (long long)nray * ncell - 1;
+    const int ray = (int)(rc / ncell), cs = (int)(rc - (long long)ray * ncell);
+    const double v0 = vr[3 * ray], v1 = vr[3 * ray + 1], v2 = vr[3 * ray + 2];
     const float T = A.temp[cs], chi_c = A.chi_c[cs];
     const float h_kT = (float)(M3D_H_K / (double)T);
     float chl[NF], gch[NF];
 #pragma unroll
     for (int f = 0; f < NF; f++) {
       chl[f] = 0.0f;
-      gch[f] = live ? g_chil[(size_t)f + (size_t)NF * cs] : 0.0f;
+      gch[f] = live ? g_chil[(size_t)f + (size_t)NF * rc] : 0.0f;
     }
     const float vproj = (float)((v0 * (double)A.vx[cs] + v1 * (double)A.vy[cs]) + v2 * (double)A.vz[cs]);
     const float ekt = A.e_kT[cs], ne = A.ne[cs], tothi = A.tothi[cs], starkpe = A.stark_pe[cs];
@@ -580,10 +688,16 @@ __global__ void __launch_bounds__(512, 1) k_opacity_adj(AtmosDev A, GridArgs G, 
         const bool full = __all_sync(conv, fa == 1 && fb == NF);
         const bool far = __all_sync(conv, fminf((xnear * cf.ih) * 800.0f, 9019.0f) >= 9018.5f);
         const float xmax = fmaxf(fabsf(x0), fabsf(xe)) * cf.ih;
-        if (__all_sync(conv, xmax <= 4611686018427387904.0f))
-          deposit_adj_mk<NF, true>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, full, far, Gl, Hl);
+        if (!__all_sync(conv, xmax <= 4611686018427387904.0f))
+          deposit_adj<NF>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
+        else if (far && full)
+          deposit_adj_x2<NF, true, true>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
+        else if (far)
+          deposit_adj_x2<NF, false, true>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
+        else if (full)
+          deposit_adj_x2<NF, true, false>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
         else
-          deposit_adj_mk<NF, false>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, full, far, Gl, Hl);
+          deposit_adj_x2<NF, false, false>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
         // K is proportional to S = Rij D: dK/dD = K/D + dK/dih dih/dD
         gB += Gl;
         gE -= L.lower_ev[l] * Gl;
@@ -593,12 +707,13 @@ __global__ void __launch_bounds__(512, 1) k_opacity_adj(AtmosDev A, GridArgs G, 
         if (grp.thread_rank() == 0) atomicAdd(&s_gp[sp * nline_max + l], tot);
       }
       if (live) {
-        g_lnbase[(size_t)sp * ncell + cs] += gB;
+        const size_t o = (size_t)ncell * ((size_t)ray * A.nspecies + sp) + cs;
+        p_lnbase[o] = gB;
         // D = sdl / idf
-        g_idf[(size_t)sp * ncell + cs] += gD * (-qw.D / idf);
+        p_idf[o] = gD * (-qw.D / idf);
       }
     }
-    if (live) g_ekt[cs] += gE;
+    if (live) p_ekt[rc] = gE;
   }
   __syncthreads();
   for (int sp = 0; sp < A.nspecies; sp++)
