@@ -37,6 +37,7 @@ struct NlWinDev {
   double cut_x;
   // per frequency: the active lines / continua whose window holds f, ascending
   const int *lf_ptr, *lf_idx, *cf_ptr, *cf_idx;
+  const float *lf_q;   // q of the line at f, beside lf_idx
 };
 
 // qlg_bot_profile (qlg_mod.f90:682-689) with the damping's set-up c at hand
@@ -218,10 +219,12 @@ __global__ void k_bb_line_consts(NlWinDev W, int ncell, int c0, int c1, const do
 // k_bb_line_consts (two 16-byte loads that a warp's lanes share): formed at every point,
 // with their conversions, double products and the set-up's division, and the point's
 // cell by a 64-bit division, they were two thirds of the kernel's 346 instructions a
-// point (48^3 cells, 8 lines and 2 continua, 250 frequencies: 0.46 -> 0.44 ms a
-// direction with the constants' 0.016; what is left waits on memory).
+// point.  The next point's background is loaded while this one's lines are summed; 62
+// registers at 4 blocks an SM (5 and 6 blocks spilled and took 19 and 10 % longer).
+// 48^3 cells, 8 lines and 2 continua, 250 frequencies: 0.46 -> 0.33 ms a direction with
+// the constants' 0.016.
 template <bool PRE>
-__global__ void k_bb_opacity(NlWinDev W, int ncell, int c0, int c1, const double *__restrict__ b,
+__global__ void __launch_bounds__(256, 4) k_bb_opacity(NlWinDev W, int ncell, int c0, int c1, const double *__restrict__ b,
                              const double *__restrict__ nstar, const double *__restrict__ pop_ratio,
                              const double *__restrict__ e_kT, const float *__restrict__ inv_df,
                              const float *__restrict__ vproj, const float *__restrict__ adamp,
@@ -229,11 +232,26 @@ __global__ void k_bb_opacity(NlWinDev W, int ncell, int c0, int c1, const double
                              float *__restrict__ xhat, float *__restrict__ ehat, NlSplit S,
                              const float *__restrict__ units_beta = nullptr, float units_floor = 0.0f,
                              const float *__restrict__ xin = nullptr, const float *__restrict__ ein = nullptr) {
-  for (PointWalk w(W.nf, c0); w.c < c1; w.next()) {
+  PointWalk w(W.nf, c0);
+  // the background from xin/ein where given (xhat/ehat then only receive the result); the
+  // next point's is loaded while this one's lines are summed
+  const float *xsrc = xin ? xin : xhat, *esrc = ein ? ein : ehat;
+  float xh1 = 0.0f, eh1 = 0.0f, be1 = 0.0f;
+  auto load = [&]() {
+    if (w.c < c1) {
+      xh1 = xsrc[w.k];
+      eh1 = esrc[w.k];
+      if (units_beta) be1 = units_beta[w.k];
+    }
+  };
+  load();
+  while (w.c < c1) {
     const size_t k = w.k;
     const int f = (int)w.f, c = w.c;
-    // the background from xin/ein where given (xhat/ehat then only receive the result)
-    float xh = xin ? xin[k] : xhat[k], eh = ein ? ein[k] : ehat[k];
+    float xh = xh1, eh = eh1;
+    const float be = be1;
+    w.next();
+    load();
     float oL = eh, oR = 0.0f, cL = xh, cR = 0.0f;
     int oid = 0, cid = 0;
     const int p0 = W.lf_ptr[f], p1 = W.lf_ptr[f + 1];
@@ -251,7 +269,7 @@ __global__ void k_bb_opacity(NlWinDev W, int ncell, int c0, int c1, const double
         } else {
           L = nl_line_const(W, ncell, c, i, b, nstar, pop_ratio, e_kT, adamp, lte);
         }
-        const float phi = nl_profile_at(tab, L.q, W.q[W.loff[i] + f - W.lblue[i]], vpr, idf);
+        const float phi = nl_profile_at(tab, L.q, W.lf_q[p], vpr, idf);
         xh = xh + phi * L.chi_fac;
         eh = eh + phi * L.eta_fac;
         if (S.sopL) {
@@ -268,7 +286,7 @@ __global__ void k_bb_opacity(NlWinDev W, int ncell, int c0, int c1, const double
     // every point leaves as chi and S
     if (units_beta) {
       float chi, Sv;
-      units_split_point(xh, units_beta[k], oL, oR, 0.0f, false, units_floor, 0, chi, Sv);
+      units_split_point(xh, be, oL, oR, 0.0f, false, units_floor, 0, chi, Sv);
       xhat[k] = chi;
       ehat[k] = Sv;
     }
@@ -341,12 +359,15 @@ constexpr int kRateWarps = 8;
 // sectors their windows share (and those a window straddles) are read from DRAM
 // once and from L2 after.  Each (line, cell) has one writer, so the order changes
 // no sum.
-// 8 cells a tile (17 KB of shared terms a block) and 64 registers give 8 blocks (32
-// warps) per SM, which hides the loads' latency better than 16-cell tiles at 6 blocks:
-// the 120^3 window's sweep 748 -> 711 ms
+// 8 cells a tile (17 KB of shared terms a block) and 48 registers give 10 blocks (40
+// warps) per SM, which hides the loads' latency better than 16-cell tiles at 6 blocks
+// (the 120^3 window's sweep 748 -> 711 ms at 8) or 8-cell ones at 8: 0.43 -> 0.41 ms a
+// direction of 48^3 cells, 8 lines and 250 frequencies, in spite of 56 bytes spilled.  Staging
+// the twelve arrays with asynchronous copies (16 warps) took 0.63 ms, two and four
+// cells' loads together 0.48-0.53, the lines' constants from a pass of their own 0.43.
 constexpr int kBbWarps = 4, kBbCells = 8;
 
-__global__ void __launch_bounds__(kBbWarps * 32, 8)
+__global__ void __launch_bounds__(kBbWarps * 32, 10)
 k_bb_rates(NlWinDev W, NlRateOpts O, int ncell, const double *__restrict__ b,
            const double *__restrict__ nstar, const double *__restrict__ pop_ratio,
            const double *__restrict__ e_kT, const float *__restrict__ inv_df,
@@ -451,22 +472,29 @@ k_bb_rates(NlWinDev W, NlRateOpts O, int ncell, const double *__restrict__ b,
             t1 = vvv * R.inu[k];
             t2 = vvv * phi * R.psi[k] * R.beta[k];
           } else {
-            const float nb = R.Bnu[k];
+            const float nb = __ldg(R.Bnu + k);
             const float vvv = phi * wmunu;
             if (O.precond) {
-              const float be = R.beta[k];
-              float psi = R.psi[k];
+              // all of the point's values before the first is used (read-only loads, which
+              // may pass the terms' stores): irem, escape and work1 are wanted wherever
+              // psi is not zero, nearly everywhere
+              const float be = __ldg(R.beta + k);
+              float psi = __ldg(R.psi + k);
+              const float sopL = __ldg(R.sopL + k), sopR = __ldg(R.sopR + k), schL = __ldg(R.schL + k);
+              const float schR = __ldg(R.schR + k);
+              const int sid = __ldg(R.sid + k), schid = __ldg(R.schid + k);
+              const float irem = __ldg(R.irem + k), escp = __ldg(R.escape + k), wk1 = __ldg(R.work1 + k);
               const float eta_u = phi * c_eta;
               const float eta_t = eta_u * be;
               const float chi_t = phi * c_abs - eta_t;
-              const float eta_other = be * other_contribution(eta_u, index, R.sopL[k], R.sopR[k], R.sid[k]);
-              const float chi_other = other_contribution(phi * c_abs, index, R.schL[k], R.schR[k], R.schid[k]) - eta_other;
+              const float eta_other = be * other_contribution(eta_u, index, sopL, sopR, sid);
+              const float chi_other = other_contribution(phi * c_abs, index, schL, schR, schid) - eta_other;
               float other = eta_other;
               if (O.do_scat) other = other + R.scat[k];
               if (chi_t < 0.0f || c_if) psi = 0.0f;
               if (psi == 0.0f) shr[wib][ci] = 1;
-              const float up = psi == 0.0f ? R.inu[k] : R.irem[k] + psi * other;
-              const float spont = psi == 0.0f ? 1.0f : (chi_other + R.escape[k] * chi_t) / R.work1[k];
+              const float up = psi == 0.0f ? R.inu[k] : irem + psi * other;
+              const float spont = psi == 0.0f ? 1.0f : (chi_other + escp * chi_t) / wk1;
               t0 = vvv * spont * (nb * c_inr);
               t1 = vvv * (up - nb * spont);
             } else {
