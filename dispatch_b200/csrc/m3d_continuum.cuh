@@ -20,11 +20,12 @@
 
 namespace m3d {
 
-constexpr int kContWarps = 4;     // warps (cells) per block
+constexpr int kContWarps = 8;     // warps per block
+constexpr int kContCells = 4;     // cells a warp works on at a time
 constexpr int kContMaxComp = 64;  // components of one call
 constexpr int kContMaxRows = 1024;  // table rows a window reads, over all components (per cell, in shared memory)
 constexpr int kContMaxTab = 8192;   // their table entries at every temperature node (per block, in shared memory)
-constexpr int kContKF = 8;          // wavelengths a lane holds in one pass over the components
+constexpr int kContKF = 1;          // wavelengths a lane holds of each cell in one pass over the components
 
 // wcalc2's per-wavelength set-up of an 'H BF' level (level_mod.f90:186-218): cls 0
 // none, 1 beyond the series limit, 2 below it (a dissolved upper level); qcut =
@@ -205,54 +206,72 @@ __device__ __forceinline__ float cont_row_s(const BfCompDev &c, const BfCellDev 
 }
 
 // one component's contributions at the lane's wavelengths f0 + 32 k (interp_xkap
-// :358-385 and :386-426), each added to v[k] where the component reaches f; l3[f]
-// is real(lambda^3).  The component's fields are read once for all of them.
-template <int KF>
-__device__ __forceinline__ void cont_comp(const BfCompDev &c, const BfCellDev &r, const float *rows, int f0,
-                                          const float *__restrict__ l3, const ContCellsDev &S, int x,
-                                          float (&v)[KF]) {
+// :358-385 and :386-426) in C cells, each added to v[cell][k] where the component reaches
+// f; l3[f] is real(lambda^3).  The component's fields are read once for all of them, the
+// wavelengths' stencils together and once for the cells: read wavelength by wavelength
+// and cell by cell, their latencies in turn were most of the kernel's time.
+// r: the component's state in each cell, rstride apart; rows: the cells' rows, sstride
+// apart; x: the cells.
+template <int KF, int C>
+__device__ __forceinline__ void cont_comp(const BfCompDev &c, const BfCellDev *r, int rstride, const float *rows,
+                                          int sstride, int f0, const float *__restrict__ l3, const ContCellsDev &S,
+                                          const int (&x)[C], float (&v)[C][KF]) {
   if (!c.active) return;
   const int fs = c.fs, fe = c.fe, nnu = c.nnu, ilogl = c.ilogl, lam3 = c.lam3;
   const float4 *wt = c.wt;
   if (c.ntt > 1) {
-    if (!r.in_bounds) return;
-    const float fakt1 = r.fakt1;
+    bool inb[C], any = false;
+#pragma unroll
+    for (int q = 0; q < C; q++) {
+      inb[q] = r[q * rstride].in_bounds;
+      any = any || inb[q];
+    }
+    if (!any) return;
     const int soff = c.soff;
     const float *yy = rows + soff - c.r0;   // yy[row], 0-based table rows
+    float4 w[KF];
+    float l[KF];
 #pragma unroll
     for (int k = 0; k < KF; k++) {
       const int f = f0 + 32 * k;
-      if (f < fs || f > fe) continue;
-      const float4 w = __ldg(wt + f);
-      const int iw = __float_as_int(w.x);
-      float ab;
-      if (iw >= 0) {
-        float y1, y2, y3;
-        if (soff >= 0) {
-          y1 = yy[iw];
-          y2 = yy[iw + 1];
-          y3 = yy[iw + 3 < nnu ? iw + 2 : nnu - 1];
+      const bool on = f >= fs && f <= fe;
+      w[k] = on ? __ldg(wt + f) : make_float4(__int_as_float(-2), 0.0f, 0.0f, 0.0f);
+      l[k] = on && lam3 ? __ldg(l3 + f) : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < KF; k++) {
+      const int iw = __float_as_int(w[k].x);   // -1: no stencil there, -2: not reached
+      if (iw == -2) continue;
+#pragma unroll
+      for (int q = 0; q < C; q++) {
+        if (!inb[q]) continue;
+        float ab;
+        if (iw >= 0) {
+          float y1, y2, y3;
+          if (soff >= 0) {
+            const float *yq = yy + q * sstride;
+            y1 = yq[iw];
+            y2 = yq[iw + 1];
+            y3 = yq[iw + 3 < nnu ? iw + 2 : nnu - 1];
+          } else {
+            const int i = iw + 1;
+            y1 = cont_row(c, r[q * rstride], i);
+            y2 = cont_row(c, r[q * rstride], i + 1);
+            y3 = cont_row(c, r[q * rstride], i + 2 < nnu ? i + 2 : nnu);
+          }
+          ab = __fadd_rn(__fadd_rn(__fmul_rn(y1, w[k].y), __fmul_rn(y2, w[k].z)), __fmul_rn(y3, w[k].w));
         } else {
-          const int i = iw + 1;
-          y1 = cont_row(c, r, i);
-          y2 = cont_row(c, r, i + 1);
-          y3 = cont_row(c, r, i + 2 < nnu ? i + 2 : nnu);
+          ab = ilogl ? -FLT_MAX : 0.0f;
         }
-        ab = __fadd_rn(__fadd_rn(__fmul_rn(y1, w.y), __fmul_rn(y2, w.z)), __fmul_rn(y3, w.w));
-      } else {
-        ab = ilogl ? -FLT_MAX : 0.0f;
+        if (ilogl) ab = exp4(ab);
+        if (lam3) ab = __fmul_rn(ab, l[k]);
+        v[q][k] = __fadd_rn(v[q][k], __fmul_rn(r[q * rstride].fakt1, ab));
       }
-      if (ilogl) ab = exp4(ab);
-      if (lam3) ab = __fmul_rn(ab, __ldg(l3 + f));
-      v[k] = __fadd_rn(v[k], __fmul_rn(fakt1, ab));
     }
   } else if (c.occ) {
     // interp_xkap_2's table at the window, then wcalc2 for the cell (bftrans_mod.f90
     // :398-428, level_mod.f90:220-277): w, 1 - w, the level's population and
     // 4 pi/3 n_H of the cell are in r; shield, ne and 4 pi/3 n_He are the cell's
-    const float w = r.w0, omw = r.w1, n = r.w2, nh43 = r.fakt1;
-    const double xd = S.shield[x];
-    const float xs = (float)xd, ne1 = (float)S.ne[x], nhe43 = (float)(4.18879 * S.nHeI[x]);
     const float *xk = c.xkap;
     const unsigned char *quad = c.quad;
     const OccFDev *occf = c.occf;
@@ -278,30 +297,36 @@ __device__ __forceinline__ void cont_comp(const BfCompDev &c, const BfCellDev &r
       if (lam3) ab = __fmul_rn(ab, __ldg(l3 + f));
       // g = real(2.0898E-26/(2 i^5) * cutfac * ab, 4), ab times real(xkap_scale, 4)
       const float g = (float)(o.qcut * (double)__fmul_rn(ab, scale));
-      float d;
-      if (o.cls == 1) {
-        d = w;
-      } else {
-        // neutral perturbers E = exp(-a); charged ones C = frac/(1+frac), tested on
-        // the real(8) product; w - wstar formed as (1 - wstar) - (1 - w) near w = 1
-        const float a = __fadd_rn(__fmul_rn(nh43, o.x1), __fmul_rn(nhe43, o.x2));
-        float E, omE;
-        exp_neg0(a, E, omE);
-        const float k1 = o.kk;
-        const float xkk = __fmul_rn(xs, k1);
-        float C = 1.0f, omC = 0.0f;
-        if (xd * o.kd < 1e4) {
-          const float den = __fadd_rn(1.0f, __fmul_rn(0.1285f, xkk));
-          const float frac = __fdiv_rn(__fmul_rn(__fmul_rn(0.1402f, xkk), k1), __fmul_rn(ne1, den));
-          C = __fdiv_rn(frac, __fadd_rn(1.0f, frac));
-          omC = __fdiv_rn(1.0f, __fadd_rn(1.0f, frac));
+#pragma unroll
+      for (int q = 0; q < C; q++) {
+        const BfCellDev &rq = r[q * rstride];
+        const float w = rq.w0, omw = rq.w1;
+        float d;
+        if (o.cls == 1) {
+          d = w;
+        } else {
+          // neutral perturbers E = exp(-a); charged ones C = frac/(1+frac), tested on
+          // the real(8) product; w - wstar formed as (1 - wstar) - (1 - w) near w = 1
+          const double xd = S.shield[x[q]];
+          const float xs = (float)xd, ne1 = (float)S.ne[x[q]], nhe43 = (float)(4.18879 * S.nHeI[x[q]]);
+          const float a = __fadd_rn(__fmul_rn(rq.fakt1, o.x1), __fmul_rn(nhe43, o.x2));
+          float E, omE;
+          exp_neg0(a, E, omE);
+          const float k1 = o.kk;
+          const float xkk = __fmul_rn(xs, k1);
+          float Cc = 1.0f, omC = 0.0f;
+          if (xd * o.kd < 1e4) {
+            const float den = __fadd_rn(1.0f, __fmul_rn(0.1285f, xkk));
+            const float frac = __fdiv_rn(__fmul_rn(__fmul_rn(0.1402f, xkk), k1), __fmul_rn(ne1, den));
+            Cc = __fdiv_rn(frac, __fadd_rn(1.0f, frac));
+            omC = __fdiv_rn(1.0f, __fadd_rn(1.0f, frac));
+          }
+          d = (w > 0.5f) ? __fsub_rn(__fadd_rn(omE, __fmul_rn(E, omC)), omw) : __fsub_rn(w, __fmul_rn(E, Cc));
         }
-        d = (w > 0.5f) ? __fsub_rn(__fadd_rn(omE, __fmul_rn(E, omC)), omw) : __fsub_rn(w, __fmul_rn(E, C));
+        v[q][k] = __fadd_rn(v[q][k], __fmul_rn(__fmul_rn(d, rq.w2), g));
       }
-      v[k] = __fadd_rn(v[k], __fmul_rn(__fmul_rn(d, n), g));
     }
   } else {
-    const float fakt1 = r.fakt1;
     const float *xk = c.xkap;
     const unsigned char *quad = c.quad;
 #pragma unroll
@@ -310,6 +335,7 @@ __device__ __forceinline__ void cont_comp(const BfCompDev &c, const BfCellDev &r
       if (f < fs || f > fe) continue;
       const float4 w = __ldg(wt + f);
       const int iw = __float_as_int(w.x);
+      // without temperature dependence the table's value is the same in every cell
       float ab;
       if (iw < 0) {
         ab = 0.0f;
@@ -321,7 +347,8 @@ __device__ __forceinline__ void cont_comp(const BfCompDev &c, const BfCellDev &r
         if (ilogl) ab = expf(ab);
       }
       if (lam3) ab = __fmul_rn(ab, __ldg(l3 + f));
-      v[k] = __fadd_rn(v[k], __fmul_rn(ab, fakt1));
+#pragma unroll
+      for (int q = 0; q < C; q++) v[q][k] = __fadd_rn(v[q][k], __fmul_rn(ab, r[q * rstride].fakt1));
     }
   }
 }
@@ -361,21 +388,36 @@ __global__ void k_continuum_lam(int nlam, const double *__restrict__ lam, int he
   he_o[f] = he;
 }
 
-// eight blocks per SM (64 registers): the latency of the stencil loads is hidden by
-// occupancy, measured faster than 80 registers at six blocks and than 56 or 48 at
-// nine or ten
-__global__ void __launch_bounds__(kContWarps * 32, 8)
+// The per-cell scalars of the wavelength loop, in shared memory
+struct ContCellLoc { double hrest, hk_T, nHI, nHe, nH2, els; };
+
+// shared memory beside the components' descriptors, the staged table entries and each
+// warp's rows: per warp and cell the scalars and the components' states
+__host__ __device__ inline size_t cont_cell_bytes(int ncomp) {
+  return kContWarps * kContCells * (sizeof(ContCellLoc) + sizeof(BfCellDev) * (size_t)ncomp);
+}
+
+// A warp takes four neighbouring cells: their components' temperature stencils and factors
+// side by side in its lanes, their rows in one pass, and each wavelength's stencil,
+// Gaunt-like table value and Rayleigh terms read once for all.  64 registers at four
+// blocks of eight warps per SM, so the window's table rows are staged four times an SM
+// instead of eight and L1 keeps the stencils.  262144 cells, 250 wavelengths, fourteen
+// components: 3.76 -> 2.49 ms against a cell a warp with eight wavelengths a lane (two
+// cells and two wavelengths 2.66, three and two 2.55, four and two 3.08 with spills, six
+// and one 2.74).
+__global__ void __launch_bounds__(kContWarps * 32, 4)
 k_continuum(int ncomp, const BfCompDev *__restrict__ comps_g, int any_istim, int nlam, ContLamDev LW,
             const double *__restrict__ nu, int ncell, ContCellsDev S, const float *__restrict__ beta,
             float *__restrict__ xhat, float *__restrict__ sigma, int rows_used, int tab_used) {
-  __shared__ BfCellDev sc[kContWarps][kContMaxComp];
+  constexpr int C = kContCells;
   extern __shared__ __align__(16) float cont_sh[];
   BfCompDev *scomp = reinterpret_cast<BfCompDev *>(cont_sh);   // (ncomp) the components' descriptors
-  float *cont_dyn = cont_sh + ncomp * (sizeof(BfCompDev) / sizeof(float));
-  float *stab = cont_dyn;                                        // (tab_used) the staged table entries
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  BfCellDev *st = sc[wib];
-  float *rows = cont_dyn + tab_used + (size_t)wib * rows_used;   // (rows_used) this cell's rows
+  ContCellLoc *loc = reinterpret_cast<ContCellLoc *>(scomp + ncomp) + wib * C;
+  BfCellDev *st = reinterpret_cast<BfCellDev *>(reinterpret_cast<ContCellLoc *>(scomp + ncomp) + kContWarps * C) +
+                  (size_t)wib * C * ncomp;
+  float *stab = reinterpret_cast<float *>(reinterpret_cast<char *>(scomp + ncomp) + cont_cell_bytes(ncomp));
+  float *rows = stab + tab_used + (size_t)wib * C * rows_used;   // (C, rows_used) the cells' rows
   {
     const int nw = ncomp * (int)(sizeof(BfCompDev) / sizeof(int));
     const int *src = reinterpret_cast<const int *>(comps_g);
@@ -397,13 +439,20 @@ k_continuum(int ncomp, const BfCompDev *__restrict__ comps_g, int any_istim, int
   __syncthreads();
   const int nwarp = gridDim.x * kContWarps;
   const double thomson = cont_thomson();
-  for (int x = blockIdx.x * kContWarps + wib; x < ncell; x += nwarp) {
-    const double temp = S.temp[x], teta = S.teta[x];
-    for (int j = lane; j < ncomp; j += 32) {
+  for (int x0 = (blockIdx.x * kContWarps + wib) * C; x0 < ncell; x0 += nwarp * C) {
+    // a last cell without a neighbour is worked on twice and written once
+    int x[C];
+#pragma unroll
+    for (int q = 0; q < C; q++) x[q] = min(x0 + q, ncell - 1);
+    const int ncl = min(C, ncell - x0);
+    // a (component, cell) per lane
+    for (int t = lane; t < C * ncomp; t += 32) {
+      const int cq = t / ncomp, j = t - cq * ncomp;
+      const int xc = min(x0 + cq, ncell - 1);
       const BfCompDev &c = comps[j];
       BfCellDev r;
       if (c.ntt > 1) {
-        r = cont_tstencil(c, temp, teta);
+        r = cont_tstencil(c, S.temp[xc], S.teta[xc]);
       } else {
         r.w0 = r.w1 = r.w2 = 0.0f;
         r.it = 0;
@@ -413,87 +462,111 @@ k_continuum(int ncomp, const BfCompDev *__restrict__ comps_g, int any_istim, int
       }
       if (c.occ && c.ntt == 1) {
         // wcalc2's per-cell terms (level_mod.f90:222-229)
-        const double wo = c.active ? c.level_w[x] : 0.0;
+        const double wo = c.active ? c.level_w[xc] : 0.0;
         r.w0 = (float)wo;
         r.w1 = (float)(1.0 - wo);
-        r.w2 = c.active ? (float)c.level_n[x] : 0.0f;
-        r.fakt1 = c.active ? (float)(4.18879 * c.n[x]) : 0.0f;
+        r.w2 = c.active ? (float)c.level_n[xc] : 0.0f;
+        r.fakt1 = c.active ? (float)(4.18879 * c.n[xc]) : 0.0f;
       } else {
-        r.fakt1 = (c.active && r.in_bounds) ? cont_factor(c, S, x) : 0.0f;
+        r.fakt1 = (c.active && r.in_bounds) ? cont_factor(c, S, xc) : 0.0f;
       }
-      st[j] = r;
+      st[t] = r;
+    }
+    // add_hrest: the H I levels above n = 15, up to the lowered ionisation limit; a cell
+    // per lane with its other scalars (hrest = 0 where it is off: 0 lambda^3 adds nothing
+    // to the zero the sum starts from)
+    if (lane < C) {
+      const int xc = min(x0 + lane, ncell - 1);
+      const double ekt = S.e_kT[xc], dxi = S.dxi[xc];
+      const double nniv2 = (double)(15.5f * 15.5f);
+      double hrest = 0.0;
+      if (S.nHI && 13.598434 >= nniv2 * dxi) {
+        double fakt = exp(-ekt * (S.HI_xion - dxi) - S.partHI[xc]);
+        fakt = (double)2.0898e-26f / (2 * 13.598434 * ekt) * fakt * S.nHI[xc];
+        hrest = exp(ekt * (13.598434 / nniv2 - dxi));
+        hrest = fakt * (hrest - 1);
+      }
+      ContCellLoc l;
+      l.hrest = hrest;
+      l.hk_T = (6.626176e-27 / 1.380662e-16) / S.temp[xc];
+      l.nHI = S.nHI ? S.nHI[xc] : 0.0;
+      l.nHe = S.nHeI ? S.nHeI[xc] : 0.0;
+      l.nH2 = S.nH2 ? S.nH2[xc] : 0.0;
+      l.els = sigma ? thomson * S.ne[xc] : 0.0;
+      loc[lane] = l;
     }
     __syncwarp();
-    // the table rows at the cell's temperature, each formed once (interp_xkap's yy)
+    // the table rows at the cells' temperatures, each formed once (interp_xkap's yy)
     for (int j = 0; j < ncomp; j++) {
       const BfCompDev &c = comps[j];
-      if (c.soff < 0 || !c.active || !st[j].in_bounds) continue;
-      for (int q = lane; q < c.nrow; q += 32) rows[c.soff + q] = cont_row_s(c, st[j], stab, c.r0 + q + 1);
+      if (c.soff < 0 || !c.active) continue;
+      for (int t = lane; t < C * c.nrow; t += 32) {
+        const int cq = t / c.nrow, q = t - cq * c.nrow;
+        if (st[cq * ncomp + j].in_bounds)
+          rows[cq * rows_used + c.soff + q] = cont_row_s(c, st[cq * ncomp + j], stab, c.r0 + q + 1);
+      }
     }
     __syncwarp();
-    // add_hrest: the H I levels above n = 15, up to the lowered ionisation limit
-    const double ekt = S.e_kT[x], dxi = S.dxi[x];
-    const double nniv2 = (double)(15.5f * 15.5f);
-    bool hrest_on = false;
-    double hrest = 0.0;
-    if (S.nHI && 13.598434 >= nniv2 * dxi) {
-      double fakt = exp(-ekt * (S.HI_xion - dxi) - S.partHI[x]);
-      fakt = (double)2.0898e-26f / (2 * 13.598434 * ekt) * fakt * S.nHI[x];
-      hrest = exp(ekt * (13.598434 / nniv2 - dxi));
-      hrest = fakt * (hrest - 1);
-      hrest_on = true;
-    }
-    const double hk_T = (6.626176e-27 / 1.380662e-16) / temp;
-    const double nHIr = S.nHI ? S.nHI[x] : 0.0, nHE = S.nHeI ? S.nHeI[x] : 0.0, nH2 = S.nH2 ? S.nH2[x] : 0.0;
-    const double els = sigma ? thomson * S.ne[x] : 0.0;
     for (int f0 = lane; f0 - lane < nlam; f0 += 32 * kContKF) {
-      float v[kContKF];
+      float v[C][kContKF];
 #pragma unroll
       for (int k = 0; k < kContKF; k++) {
         const int f = f0 + 32 * k;
-        v[k] = (hrest_on && f < nlam) ? (float)((double)0.0f + hrest * __ldg(LW.cube + f)) : 0.0f;
+        const double c3 = f < nlam ? __ldg(LW.cube + f) : 0.0;
+#pragma unroll
+        for (int q = 0; q < C; q++) v[q][k] = (float)((double)0.0f + loc[q].hrest * c3);
       }
       for (int j = 0; j < ncomp; j++) {
         const BfCompDev &c = comps[j];
-        if (!c.istim) cont_comp<kContKF>(c, st[j], rows, f0, LW.l3, S, x, v);
+        if (!c.istim) cont_comp<kContKF, C>(c, st + j, ncomp, rows, rows_used, f0, LW.l3, S, x, v);
       }
       if (any_istim) {
-        float tmp[kContKF];
+        float tmp[C][kContKF];
 #pragma unroll
-        for (int k = 0; k < kContKF; k++) tmp[k] = 0.0f;
+        for (int q = 0; q < C; q++)
+#pragma unroll
+          for (int k = 0; k < kContKF; k++) tmp[q][k] = 0.0f;
         for (int j = 0; j < ncomp; j++) {
           const BfCompDev &c = comps[j];
-          if (c.istim) cont_comp<kContKF>(c, st[j], rows, f0, LW.l3, S, x, tmp);
+          if (c.istim) cont_comp<kContKF, C>(c, st + j, ncomp, rows, rows_used, f0, LW.l3, S, x, tmp);
         }
 #pragma unroll
         for (int k = 0; k < kContKF; k++) {
           const int f = f0 + 32 * k;
           if (f >= nlam) break;
-          float b;
-          if (beta) {
-            b = beta[(size_t)f + (size_t)nlam * x];
-          } else {
-            b = (float)exp(-nu[f] * hk_T);
-            b = b > FLT_MIN ? b : FLT_MIN;
+#pragma unroll
+          for (int q = 0; q < C; q++) {
+            float b;
+            if (beta) {
+              b = beta[(size_t)f + (size_t)nlam * x[q]];
+            } else {
+              b = (float)exp(-nu[f] * loc[q].hk_T);
+              b = b > FLT_MIN ? b : FLT_MIN;
+            }
+            v[q][k] = __fadd_rn(v[q][k], __fdiv_rn(tmp[q][k], __fsub_rn(1.0f, b)));
           }
-          v[k] = __fadd_rn(v[k], __fdiv_rn(tmp[k], __fsub_rn(1.0f, b)));
         }
       }
 #pragma unroll
       for (int k = 0; k < kContKF; k++) {
         const int f = f0 + 32 * k;
         if (f >= nlam) break;
-        const size_t o = (size_t)f + (size_t)nlam * x;
-        xhat[o] = v[k];
-        if (sigma) {
-          float s = (float)(0.0 + els);
-          const double xr = __ldg(LW.xr + f);
-          if (xr > 0.) {
-            const double rayh = __ldg(LW.rayh + f) * nHIr;
-            const double rayh2 = __ldg(LW.rayh2 + f) * nH2;
-            s = (float)((double)s + (rayh + rayh2) * xr * xr);
+        const double xr = sigma ? __ldg(LW.xr + f) : 0.0, rh = sigma ? __ldg(LW.rayh + f) : 0.0;
+        const double rh2 = sigma ? __ldg(LW.rayh2 + f) : 0.0, he = sigma ? __ldg(LW.he + f) : 0.0;
+#pragma unroll
+        for (int q = 0; q < C; q++) {
+          if (q >= ncl) break;
+          const size_t o = (size_t)f + (size_t)nlam * x[q];
+          xhat[o] = v[q][k];
+          if (sigma) {
+            float s = (float)(0.0 + loc[q].els);
+            if (xr > 0.) {
+              const double rayh = rh * loc[q].nHI;
+              const double rayh2 = rh2 * loc[q].nH2;
+              s = (float)((double)s + (rayh + rayh2) * xr * xr);
+            }
+            sigma[o] = (float)((double)s + he * loc[q].nHe);
           }
-          sigma[o] = (float)((double)s + __ldg(LW.he + f) * nHE);
         }
       }
     }
