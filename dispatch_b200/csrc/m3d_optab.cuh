@@ -103,158 +103,226 @@ __device__ __forceinline__ void optab_cell(const OptabDev &T, double temp, doubl
   je = (int)ife - 1;
 }
 
-// collapse (optab_mod.f90:251-286): wavelength at the four (temp, ne) corners,
-// the PC slopes carried across it, then temp, then ne
-__device__ __forceinline__ float optab_collapse(const float4 *t, size_t base, size_t sit, size_t sje, const float w[5],
-                                                const float tc[5], const float nc[5]) {
-  const float pl = w[0], opl = 1.0f - pl;
-  float v[4], gt[4], ge[4];
-#pragma unroll
-  for (int c = 0; c < 4; c++) {
-    const size_t a = base + (c & 1) * sit + (c >> 1) * sje;
-    const float4 A = __ldg(t + a), B = __ldg(t + a + 1);
-    v[c] = fmaf(w[4], B.y, fmaf(w[3], A.y, fmaf(w[2], B.x, w[1] * A.x)));
-    gt[c] = fmaf(pl, B.z, opl * A.z);
-    ge[c] = fmaf(pl, B.w, opl * A.w);
-  }
-  const float pt = tc[0], opt = 1.0f - pt;
-  const float f0 = fmaf(tc[4], gt[1], fmaf(tc[3], gt[0], fmaf(tc[2], v[1], tc[1] * v[0])));
-  const float f1 = fmaf(tc[4], gt[3], fmaf(tc[3], gt[2], fmaf(tc[2], v[3], tc[1] * v[2])));
-  const float ge0 = fmaf(pt, ge[1], opt * ge[0]);
-  const float ge1 = fmaf(pt, ge[3], opt * ge[2]);
-  return fmaf(nc[4], ge1, fmaf(nc[3], ge0, fmaf(nc[2], f1, nc[1] * f0)));
+// What a cell's queries share, formed by one lane and read by all: the PC coordinates'
+// Hermite coefficients (p, 1 - p, cm0, cm1), the table's first node at (it, je), chi500
+// and the velocity factor
+struct OptabCell {
+  float4 tc, nc;
+  long long base;
+  double vf;
+  float ch;
+};
+
+__device__ __forceinline__ OptabCell optab_cell_of(const OptabDev &T, double temp, double ne, float ch, double vf) {
+  int it, je;
+  float tc[5], nc[5];
+  optab_cell(T, temp, ne, it, je, tc, nc);
+  OptabCell r;
+  r.tc = make_float4(tc[0], tc[1], tc[3], tc[4]);
+  r.nc = make_float4(nc[0], nc[1], nc[3], nc[4]);
+  r.base = (long long)it * T.nnu + (long long)je * T.nnu * T.ntemp;
+  r.vf = vf;
+  r.ch = ch;
+  return r;
 }
 
-// the collapse of a query on node n: the node's value and PC slopes at the four
-// (temp, ne) corners, then temp, then ne, as optab_collapse forms them
-__device__ __forceinline__ float optab_collapse_node(const float4 *t, size_t base, size_t sit, size_t sje,
-                                                     const float tc[5], const float nc[5]) {
+// collapse (optab_mod.f90:251-286), its PC part: v the wavelength collapses and gt, ge the
+// PC slopes at the four (temp, ne) corners; temp, then ne
+__device__ __forceinline__ float optab_collapse_pc(const float (&v)[4], const float (&gt)[4], const float (&ge)[4],
+                                                   const float4 tc, const float4 nc) {
+  const float f0 = fmaf(tc.w, gt[1], fmaf(tc.z, gt[0], fmaf(tc.x, v[1], tc.y * v[0])));
+  const float f1 = fmaf(tc.w, gt[3], fmaf(tc.z, gt[2], fmaf(tc.x, v[3], tc.y * v[2])));
+  const float ge0 = fmaf(tc.x, ge[1], tc.y * ge[0]);
+  const float ge1 = fmaf(tc.x, ge[3], tc.y * ge[2]);
+  return fmaf(nc.w, ge1, fmaf(nc.z, ge0, fmaf(nc.x, f1, nc.y * f0)));
+}
+
+// the wavelength's part at corner nodes A and B = A + 1, weights w = (p, cm0, cm1)
+__device__ __forceinline__ float optab_collapse(const float4 (&A)[4], const float4 (&B)[4], float p, float cm0,
+                                                float cm1, const float4 tc, const float4 nc) {
+  const float op = 1.0f - p;
   float v[4], gt[4], ge[4];
 #pragma unroll
   for (int c = 0; c < 4; c++) {
-    const float4 A = __ldg(t + base + (c & 1) * sit + (c >> 1) * sje);
-    v[c] = A.x;
-    gt[c] = A.z;
-    ge[c] = A.w;
+    v[c] = fmaf(cm1, B[c].y, fmaf(cm0, A[c].y, fmaf(p, B[c].x, op * A[c].x)));
+    gt[c] = fmaf(p, B[c].z, op * A[c].z);
+    ge[c] = fmaf(p, B[c].w, op * A[c].w);
   }
-  const float pt = tc[0], opt = 1.0f - pt;
-  const float f0 = fmaf(tc[4], gt[1], fmaf(tc[3], gt[0], fmaf(tc[2], v[1], tc[1] * v[0])));
-  const float f1 = fmaf(tc[4], gt[3], fmaf(tc[3], gt[2], fmaf(tc[2], v[3], tc[1] * v[2])));
-  const float ge0 = fmaf(pt, ge[1], opt * ge[0]);
-  const float ge1 = fmaf(pt, ge[3], opt * ge[2]);
-  return fmaf(nc[4], ge1, fmaf(nc[3], ge0, fmaf(nc[2], f1, nc[1] * f0)));
+  return optab_collapse_pc(v, gt, ge, tc, nc);
+}
+
+// the collapse of a query on a node: the node's value and PC slopes at the four corners
+__device__ __forceinline__ float optab_collapse_node(const float4 (&A)[4], const float4 tc, const float4 nc) {
+  float v[4], gt[4], ge[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    v[c] = A[c].x;
+    gt[c] = A[c].z;
+    ge[c] = A[c].w;
+  }
+  return optab_collapse_pc(v, gt, ge, tc, nc);
+}
+
+// the nodes of wavelength node k at the four (temp, ne) corners
+__device__ __forceinline__ void optab_corners(const float4 *t, long long at, int sit, long long sje, float4 (&A)[4]) {
+#pragma unroll
+  for (int c = 0; c < 4; c++) A[c] = __ldg(t + at + (c & 1) * sit + (c >> 1) * sje);
 }
 
 constexpr int kOptabWarps = 8;
-// both samplers are latency-bound: at most 64 registers give 4 blocks (32 warps) per
-// SM, measured faster than 66-77 registers at 3 blocks and than 48 or 40 with spills
-constexpr int kOptabMinBlocks = 4;
-constexpr int kOptabUnroll = 1;   // frequencies per lane per pass of sample_interpolate_ll
-constexpr int kOptabLLMinBlocks = 4;   // 5 or 6 spill and are slower
+// Both samplers take kOptabCells neighbouring cells a warp and keep the table nodes of the
+// last one in registers: neighbours in a row mostly lie in one (T, ne) cell of the table,
+// and with the line list's shifts mostly between the same wavelength nodes, so a lane
+// rereads its nodes only where they differ.  A cell at a time, the nodes' 16-byte loads
+// kept the L1 data pipe 77 and 71 % busy.  64^3 cells of a cube, 256 frequencies:
+// 0.44 -> 0.25 and 1.17 -> 1.02 ms.
+// Cells a warp and registers were chosen together, by time: 8 cells at 80 registers (4 at
+// 64: 0.33 ms, 8 at 122: 0.28, 16 at 122: 0.27), for the line list 4 at 128 (2: 1.32, 3:
+// 1.11, 6: 1.43, 4 at 80 with spills: 1.71); its cells' work slots read only where they are
+// added to took 1.9.
+constexpr int kOptabCells = 8, kOptabCellsLL = 4;
 
-// sample_interpolate (optab_mod.f90:181-287): one warp per cell, lanes over the
-// frequencies; back = (kappa + kappa_scat) chi500, scat = kappa_scat chi500
-__global__ void __launch_bounds__(32 * kOptabWarps, kOptabMinBlocks) k_optab_sample(OptabDev T, int nf, long long ncell,
+// sample_interpolate (optab_mod.f90:181-287), lanes over the frequencies; back = (kappa +
+// kappa_scat) chi500, scat = kappa_scat chi500
+__global__ void __launch_bounds__(32 * kOptabWarps, 3) k_optab_sample(OptabDev T, int nf, long long ncell,
                                                                    const double *temp, const double *ne,
                                                                    const float *chi500, const OptabFreq *fc,
                                                                    float *back, float *scat) {
-  const int lane = threadIdx.x & 31;
-  const long long w0 = (long long)blockIdx.x * kOptabWarps + (threadIdx.x >> 5);
-  const long long nw = (long long)gridDim.x * kOptabWarps;
-  const size_t sit = (size_t)T.nnu, sje = (size_t)T.nnu * T.ntemp;
-  for (long long c = w0; c < ncell; c += nw) {
-    int it, je;
-    float tc[5], nc[5];
-    optab_cell(T, temp[c], ne[c], it, je, tc, nc);
-    const float ch = chi500[c];
-    const size_t cb = (size_t)it * sit + (size_t)je * sje;
+  constexpr int G = kOptabCells;
+  __shared__ OptabCell cells[kOptabWarps][G];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const long long w0 = (long long)blockIdx.x * kOptabWarps + wib, nw = (long long)gridDim.x * kOptabWarps;
+  const int sit = T.nnu;
+  const long long sje = (long long)T.nnu * T.ntemp;
+  for (long long c0 = w0 * G; c0 < ncell; c0 += nw * G) {
+    const int ncl = (int)min((long long)G, ncell - c0);
+    if (lane < ncl) cells[wib][lane] = optab_cell_of(T, temp[c0 + lane], ne[c0 + lane], chi500[c0 + lane], 1.0);
+    __syncwarp();
     for (int f = lane; f < nf; f += 32) {
-      const OptabFreq q = fc[f];
-      float kap, kas;
-      if (q.node >= 0) {
-        kap = optab_collapse_node(T.tv, cb + q.node, sit, sje, tc, nc);
-        kas = optab_collapse_node(T.ts, cb + q.node, sit, sje, tc, nc);
-      } else {
-        const float w[5] = {q.pl, q.wc0, q.wc1, q.wcm0, q.wcm1};
-        kap = optab_collapse(T.tv, cb + q.k, sit, sje, w, tc, nc);
-        kas = optab_collapse(T.ts, cb + q.k, sit, sje, w, tc, nc);
+      const int node = fc[f].node;
+      const int k = node >= 0 ? node : fc[f].k;
+      float4 A[4], As[4];
+      long long base = -1;
+#pragma unroll
+      for (int g = 0; g < G; g++) {
+        if (g >= ncl) break;
+        const OptabCell &q = cells[wib][g];
+        if (q.base != base) {
+          base = q.base;
+          optab_corners(T.tv, base + k, sit, sje, A);
+          optab_corners(T.ts, base + k, sit, sje, As);
+        }
+        float kap, kas;
+        if (node >= 0) {
+          kap = optab_collapse_node(A, q.tc, q.nc);
+          kas = optab_collapse_node(As, q.tc, q.nc);
+        } else {
+          const OptabFreq w = fc[f];
+          float4 B[4];
+          optab_corners(T.tv, base + k + 1, sit, sje, B);
+          kap = optab_collapse(A, B, w.pl, w.wcm0, w.wcm1, q.tc, q.nc);
+          optab_corners(T.ts, base + k + 1, sit, sje, B);
+          kas = optab_collapse(As, B, w.pl, w.wcm0, w.wcm1, q.tc, q.nc);
+        }
+        const size_t o = (size_t)(c0 + g) * nf + f;
+        back[o] = (kap + kas) * q.ch;
+        scat[o] = kas * q.ch;
       }
-      const size_t o = (size_t)c * nf + f;
-      back[o] = (kap + kas) * ch;
-      scat[o] = kas * ch;
     }
+    __syncwarp();
   }
 }
 
 // sample_interpolate_ll (optab_mod.f90:300-409): the query wavelength of each
-// cell is lam_q (1 + vproj), bracketed by walking from the unshifted count;
-// xhat, ehat += kappa chi500, and chi_scat += kappa_scat chi500 when given.
-// A lane takes kOptabUnroll frequencies per pass: their work slots are read and
-// their brackets found before the table lookups.  One frequency at 4 blocks per SM
-// measured faster (8.7 ms at 2.1 M cells x 256) than two (10.6 ms), which held the
-// reads of two in flight at the cost of registers.
-__global__ void __launch_bounds__(32 * kOptabWarps, kOptabLLMinBlocks) k_optab_sample_ll(OptabDev T, int nf, long long ncell,
+// cell is lam_q (1 + vproj), bracketed by walking from its neighbour's count (the
+// unshifted one for the first); xhat, ehat += kappa chi500, and chi_scat += kappa_scat
+// chi500 when given.
+__global__ void __launch_bounds__(32 * kOptabWarps, 2) k_optab_sample_ll(OptabDev T, int nf, long long ncell,
                                                                       const double *temp, const double *ne,
                                                                       const float *chi500, const float *vproj,
                                                                       const double *lam_q, const OptabFreq *fc,
                                                                       float *xhat, float *ehat, float *chi_scat) {
-  const int lane = threadIdx.x & 31;
-  const long long w0 = (long long)blockIdx.x * kOptabWarps + (threadIdx.x >> 5);
-  const long long nw = (long long)gridDim.x * kOptabWarps;
-  const size_t sit = (size_t)T.nnu, sje = (size_t)T.nnu * T.ntemp;
-  const int nnu = T.nnu;
+  constexpr int G = kOptabCellsLL;
+  __shared__ OptabCell cells[kOptabWarps][G];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const long long w0 = (long long)blockIdx.x * kOptabWarps + wib, nw = (long long)gridDim.x * kOptabWarps;
+  const int sit = T.nnu, nnu = T.nnu;
+  const long long sje = (long long)T.nnu * T.ntemp;
   const double *lam = T.lam;
-  for (long long c = w0; c < ncell; c += nw) {
-    int it, je;
-    float tc[5], nc[5];
-    optab_cell(T, temp[c], ne[c], it, je, tc, nc);
-    const float ch = chi500[c];
-    const double vf = 1.0 + (double)vproj[c];
-    const size_t cb = (size_t)it * sit + (size_t)je * sje;
-    for (int f0 = lane; f0 < nf; f0 += 32 * kOptabUnroll) {
-      float xv[kOptabUnroll], ev[kOptabUnroll], sv[kOptabUnroll];
-      int k[kOptabUnroll], nd[kOptabUnroll];
-      float w[kOptabUnroll][5];
+  for (long long c0 = w0 * G; c0 < ncell; c0 += nw * G) {
+    const int ncl = (int)min((long long)G, ncell - c0);
+    if (lane < ncl)
+      cells[wib][lane] = optab_cell_of(T, temp[c0 + lane], ne[c0 + lane], chi500[c0 + lane],
+                                       1.0 + (double)vproj[c0 + lane]);
+    __syncwarp();
+    for (int f = lane; f < nf; f += 32) {
+      const double lq = lam_q[f];
+      int cnt = fc[f].cnt;
+      // the nodes on either side of the count stay at hand: a neighbour's query mostly
+      // falls between the same two
+      double llo = cnt > 0 ? lam[cnt - 1] : -HUGE_VAL, lhi = cnt < nnu ? lam[cnt] : HUGE_VAL;
+      // the work slots of every cell, then their brackets
+      float xv[G], ev[G], sv[G], p[G], cm0[G], cm1[G];
+      int k[G];
 #pragma unroll
-      for (int u = 0; u < kOptabUnroll; u++) {
-        const int f = f0 + 32 * u;
-        if (f >= nf) break;
-        const size_t o = (size_t)c * nf + f;
-        xv[u] = xhat[o];
-        ev[u] = ehat[o];
-        if (chi_scat) sv[u] = chi_scat[o];
-        const double x = __dmul_rn(lam_q[f], vf);
-        int cnt = fc[f].cnt;
-        while (cnt < nnu && lam[cnt] < x) cnt++;
-        while (cnt > 0 && lam[cnt - 1] >= x) cnt--;
-        k[u] = optab_interval(nnu, lam, cnt, x, w[u]);
-        nd[u] = optab_on_node(w[u], k[u]);
+      for (int g = 0; g < G; g++) {
+        const size_t o = (size_t)(c0 + g) * nf + f;
+        xv[g] = g < ncl ? xhat[o] : 0.0f;
+        ev[g] = g < ncl ? ehat[o] : 0.0f;
+        sv[g] = g < ncl && chi_scat ? chi_scat[o] : 0.0f;
       }
 #pragma unroll
-      for (int u = 0; u < kOptabUnroll; u++) {
-        const int f = f0 + 32 * u;
-        if (f >= nf) break;
-        const float kap = nd[u] >= 0 ? optab_collapse_node(T.tv, cb + nd[u], sit, sje, tc, nc)
-                                     : optab_collapse(T.tv, cb + k[u], sit, sje, w[u], tc, nc);
-        const float add = kap * ch;
-        xv[u] = xv[u] + add;
-        ev[u] = ev[u] + add;
-        if (chi_scat) {
-          const float kas = nd[u] >= 0 ? optab_collapse_node(T.ts, cb + nd[u], sit, sje, tc, nc)
-                                       : optab_collapse(T.ts, cb + k[u], sit, sje, w[u], tc, nc);
-          sv[u] = sv[u] + kas * ch;
+      for (int g = 0; g < G; g++) {
+        if (g >= ncl) break;
+        const double x = __dmul_rn(lq, cells[wib][g].vf);
+        while (lhi < x) {
+          cnt++;
+          llo = lhi;
+          lhi = cnt < nnu ? lam[cnt] : HUGE_VAL;
         }
+        while (llo >= x) {
+          cnt--;
+          lhi = llo;
+          llo = cnt > 0 ? lam[cnt - 1] : -HUGE_VAL;
+        }
+        float w[5];
+        k[g] = (cnt < 1 ? 1 : (cnt > nnu - 1 ? nnu - 1 : cnt)) - 1;
+        const bool inside = cnt >= 1 && cnt <= nnu - 1;
+        const double l0 = inside ? llo : lam[k[g]], l1 = inside ? lhi : lam[k[g] + 1];
+        optab_hcoefs((float)((x - l0) / (l1 - l0)), (float)(l1 - l0), w);
+        p[g] = w[0];
+        cm0[g] = w[3];
+        cm1[g] = w[4];
       }
+      auto component = [&](const float4 *t, auto add) {
+        float4 A[4], B[4];
+        long long at = -1;
 #pragma unroll
-      for (int u = 0; u < kOptabUnroll; u++) {
-        const int f = f0 + 32 * u;
-        if (f >= nf) break;
-        const size_t o = (size_t)c * nf + f;
-        xhat[o] = xv[u];
-        ehat[o] = ev[u];
-        if (chi_scat) chi_scat[o] = sv[u];
-      }
+        for (int g = 0; g < G; g++) {
+          if (g >= ncl) break;
+          const OptabCell &q = cells[wib][g];
+          if (q.base + k[g] != at) {
+            at = q.base + k[g];
+            optab_corners(t, at, sit, sje, A);
+            optab_corners(t, at + 1, sit, sje, B);
+          }
+          const float w[5] = {p[g], 1.0f - p[g], p[g], cm0[g], cm1[g]};
+          const int nd = optab_on_node(w, k[g]);
+          const float kap = nd < 0 ? optab_collapse(A, B, p[g], cm0[g], cm1[g], q.tc, q.nc)
+                            : nd == k[g] ? optab_collapse_node(A, q.tc, q.nc)
+                                         : optab_collapse_node(B, q.tc, q.nc);
+          add(g, kap * q.ch);
+        }
+      };
+      component(T.tv, [&](int g, float a) {
+        const size_t o = (size_t)(c0 + g) * nf + f;
+        xhat[o] = xv[g] + a;
+        ehat[o] = ev[g] + a;
+      });
+      if (chi_scat)
+        component(T.ts, [&](int g, float a) { chi_scat[(size_t)(c0 + g) * nf + f] = sv[g] + a; });
     }
+    __syncwarp();
   }
 }
 
