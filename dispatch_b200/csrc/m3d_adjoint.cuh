@@ -519,11 +519,11 @@ __device__ __forceinline__ void deposit_adj_x2(float (&chl)[NF], const float (&g
     f32x2 F = pk2((float)(2 * k), (float)(2 * k + 1));
     if (!FULL) F = add2(F, KF);
     const f32x2 xs = mul2(add2(X0, F), IH);
-    float xa, xb;
+    const f32x2 u = fma2(xs, xs, 0);    // as deposit_window_x2 forms it
+    const f32x2 d = add2(u, ONE), nd = fma2(u, NEG, NEG);
+    float xa, xb, da, db;
     up2(xs, xa, xb);
-    const float ua = xa * xa, ub = xb * xb;
-    const float da = 1.0f + ua, db = 1.0f + ub;
-    const f32x2 nd = pk2(-da, -db);
+    up2(d, da, db);
     const f32x2 r = pk2(rcp_approx(da), rcp_approx(db));
     const f32x2 L = fma2(r, fma2(nd, r, ONE), r);
     f32x2 P, gG, cWd, e, eg;
@@ -553,7 +553,7 @@ __device__ __forceinline__ void deposit_adj_x2(float (&chl)[NF], const float (&g
     }
     const f32x2 t = fma2(NEG, fma2(add2(L, L), P, BL), cWd);
     const f32x2 dKu = fma2(mul2(L, L), t, gG);
-    f32x2 dKi = fma2(dKu, mul2(pk2(ua, ub), R2IH), fma2(L, fma2(L, e, DBL), eg));
+    f32x2 dKi = fma2(dKu, mul2(u, R2IH), fma2(L, fma2(L, e, DBL), eg));
     if (!FULL) {
       float ka, kb, ha, hb;
       up2(K, ka, kb);

@@ -183,10 +183,11 @@ __device__ __forceinline__ void deposit_window(float (&chl)[NF], const float2 *s
 // is below 2^126 (the Markstein reciprocal).  Exact rewrites beside the packing:
 //  * xs is formed with its sign, x ih; only xs^2 and |xs| are used, and the rounded
 //    product is symmetric in the sign;
-//  * d = 1 + xs^2 is formed per half in scalar (a packed product feeding a packed
-//    sum was fused into one rounding by the code generator, which left K 1-2 ulp off
-//    at a few points of about one table-form window in 10^4), and -d enters the
-//    Newton step;
+//  * xs^2 is formed as a packed fma with +0: a packed product feeding the packed sum
+//    1 + xs^2 was fused into one rounding by the code generator, which left K 1-2 ulp
+//    off at a few points of about one table-form window in 10^4, and the two formed per
+//    half in scalar cost three more instructions a pair; -(1 + xs^2) enters the Newton
+//    step;
 //  * the snapped node nint(min(|xs| 800, 9019)) is floor(RZ(y + 0.5)): rounding
 //    toward zero never carries a positive sum past the integer below it, so this is
 //    round-half-up of y >= 0, i.e. nint, with no special case below y = 0.5.  Adding
@@ -211,7 +212,7 @@ template <int NF, bool FULL, bool FAR, bool OFF>
 __device__ __forceinline__ void deposit_window_x2(float (&chl)[NF], const float2 *s_tab, const QlgCoef &cf,
                                                   float x0, const LaneWin &w) {
   static_assert(NF % 4 == 0, "pairs of window points, in two halves");
-  const f32x2 X0 = splat2(x0), IH = splat2(cf.ih), ONE = splat2(1.0f), BL = splat2(cf.bL);
+  const f32x2 X0 = splat2(x0), IH = splat2(cf.ih), ONE = splat2(1.0f), NEG = splat2(-1.0f), BL = splat2(cf.bL);
   const f32x2 KLO = splat2(w.klo), KHI = splat2(w.khi);
   f32x2 P1 = 0, GG = 0, CZH = 0, CL2 = 0, GGc = 0;
   unsigned base = 0;
@@ -232,21 +233,23 @@ __device__ __forceinline__ void deposit_window_x2(float (&chl)[NF], const float2
     if (!FULL || OFF) F = add2(F, 2 * k >= NF / 2 ? KHI : KLO);  // exact
     const f32x2 x = add2(X0, F);
     const f32x2 xs = mul2(x, IH);
-    float xa, xb;
-    up2(xs, xa, xb);
-    // 1 + xs^2 in scalar: the code generator fuses a packed product into the packed
-    // sum that consumes it (one rounding where the reference rounds twice), which
-    // the scalar forms under -fmad=false never are
-    const float da = 1.0f + xa * xa, db = 1.0f + xb * xb;
-    const f32x2 nd = pk2(-da, -db);
-    const f32x2 r = pk2(rcp_approx(da), rcp_approx(db));
+    // xs^2 as a fused product with +0, which rounds as the product does (xs^2 is never
+    // -0) and which the code generator cannot fuse into the sum that consumes it, as it
+    // does a plain packed product (one rounding where the reference rounds twice); then
+    // 1 + xs^2 and its negative, each rounded once
+    const f32x2 u = fma2(xs, xs, 0);
+    const f32x2 nd = fma2(u, NEG, NEG);
+    float xa, xb, da, db;
+    up2(mul2(xs, splat2(800.0f)), xa, xb);
+    up2(nd, da, db);
+    const f32x2 r = pk2(rcp_approx(-da), rcp_approx(-db));
     const f32x2 e = fma2(nd, r, ONE);
     const f32x2 L = fma2(r, e, r);
     f32x2 K;
     if (FAR) {
       K = fma2(L, fma2(L, P1, BL), GG);
     } else {
-      const f32x2 y = pk2(fminf(fabsf(xa) * 800.0f, 9019.0f), fminf(fabsf(xb) * 800.0f, 9019.0f));
+      const f32x2 y = pk2(fminf(fabsf(xa), 9019.0f), fminf(fabsf(xb), 9019.0f));
       const f32x2 v = add2_rz(add2_rz(y, splat2(0.5f)), splat2(8388608.0f));
       float va, vb;
       up2(v, va, vb);
