@@ -700,7 +700,7 @@ __host__ __device__ inline size_t se_team_doubles(int n, int N) {
 // and some fifty registers beside them; the general collision forms take what they need
 __host__ __device__ constexpr int se_threads(int TEAM, int N) { return N == 0 ? 128 : TEAM == 64 ? 64 : 128; }
 __host__ __device__ constexpr int se_min_blocks(int CM, int N) {
-  return N == 0 ? (CM == 2 ? 2 : 4) : CM == 2 ? 1 : N <= 16 ? 6 : N <= 24 ? 5 : N <= 32 ? 4 : N <= 48 ? 7 : 6;
+  return N == 0 ? (CM == 2 ? 2 : 4) : CM == 2 ? 1 : N <= 24 ? 6 : N <= 32 ? 4 : N <= 48 ? 7 : 6;
 }
 
 // update_populations over all cells: warps stride over the cells in ascending order
