@@ -48,19 +48,37 @@ __device__ __forceinline__ float exp4(float x) {
   return (t <= 87.0f) ? E : 0.0f;
 }
 
-// fp32 log from the atanh series: x = 2^e m, m in [sqrt(1/2), sqrt(2)),
+// 1/d correctly rounded for d in [1, 2^126): the approximate reciprocal refined by
+// one Newton step in fused multiply-adds, e = 1 - d r, r + r e (Markstein's method,
+// IBM J. Res. Dev. 34 (1990) 111).  Equal to __frcp_rn on every float of that range
+// (an exhaustive comparison on the B200); beyond it the approximation flushes to
+// zero, so callers bound d first.
+__device__ __forceinline__ float rcp_markstein(float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float e = fmaf(-d, r, 1.0f);
+  return fmaf(r, e, r);
+}
+
+// fp32 log from the atanh series: x = 2^e m, m in (sqrt(1/2), sqrt(2)],
 // log m = 2 atanh(s), s = (m-1)/(m+1), series to s^11; e ln2 with a split ln2.
+// e comes from the bits less those of the float after sqrt(1/2).  s is the correctly
+// rounded quotient: the product by the correctly rounded reciprocal, one correction by
+// the remainder (Markstein, as rcp_markstein); equal to the division at all 2^23
+// mantissas (an exhaustive comparison).
 __device__ __forceinline__ float logf_m3d(float x) {
-  if (!(x > 0.0f)) return x == 0.0f ? -INFINITY : __int_as_float(0x7fc00000);
-  if (x == INFINITY) return x;
   int e = 0;
-  if (x < FLT_MIN) { x = x * 8388608.0f; e = -23; }
-  const uint32_t u = __float_as_uint(x);
-  e += (int)((u >> 23) & 0xff) - 127;
-  float m = __uint_as_float((u & 0x7fffffu) | 0x3f800000u);
-  if (m > 1.41421356f) { m = m * 0.5f; e += 1; }
-  const float f = m - 1.0f;
-  const float s = f / (2.0f + f);
+  if (__float_as_uint(x) - 0x00800000u >= 0x7f000000u) {   // not a normal positive number
+    if (!(x > 0.0f)) return x == 0.0f ? -INFINITY : __int_as_float(0x7fc00000);
+    if (x == INFINITY) return x;
+    x = x * 8388608.0f;
+    e = -23;
+  }
+  const int u = __float_as_int(x), k = (u - 0x3f3504f4) >> 23;
+  e += k;
+  const float f = __int_as_float(u - (k << 23)) - 1.0f;
+  const float d = 2.0f + f, rd = rcp_markstein(d), q0 = f * rd;
+  const float s = fmaf(fmaf(-q0, d, f), rd, q0);
   const float s2 = s * s;
   float p = fmaf(s2, 0.0909090936f, 0.111111112f);
   p = fmaf(s2, p, 0.142857143f);
