@@ -520,11 +520,11 @@ __device__ __forceinline__ void deposit_adj_x2(float (&chl)[NF], const float (&g
     if (!FULL) F = add2(F, KF);
     const f32x2 xs = mul2(add2(X0, F), IH);
     const f32x2 u = fma2(xs, xs, 0);    // as deposit_window_x2 forms it
-    const f32x2 d = add2(u, ONE), nd = fma2(u, NEG, NEG);
+    const f32x2 nd = fma2(u, NEG, NEG);
     float xa, xb, da, db;
     up2(xs, xa, xb);
-    up2(d, da, db);
-    const f32x2 r = pk2(rcp_approx(da), rcp_approx(db));
+    up2(nd, da, db);
+    const f32x2 r = pk2(rcp_approx(-da), rcp_approx(-db));
     const f32x2 L = fma2(r, fma2(nd, r, ONE), r);
     f32x2 P, gG, cWd, e, eg;
     f32x2 K;
@@ -643,12 +643,17 @@ __global__ void __launch_bounds__(512, 1) k_opacity_adj(AtmosDev A, GridArgs G, 
       const float lvb2 = logf_m3d(Sd.vbar2[cs]);
       const float unsold_c = exp4(0.3f * lvb2) * tothi;
       float gB = 0.0f, gD = 0.0f;
-      for (int l = 0; l < L.nline; l++) {
-        if (L.active && !L.active[l]) continue;
-        const float ex = L.lower_ev[l] * ekt;
-        const float arg = (base + L.gpref[l]) - ex;
+      const LineRec *rec = L.rec;
+      const int nline = L.nline;
+      for (int l = 0; l < nline; l++) {
+        double llam0;
+        float lower_ev, gpref;
+        line_place(rec + l, llam0, lower_ev, gpref);
+        if (__float_as_uint(gpref) == LINE_OFF) continue;
+        const float ex = lower_ev * ekt;
+        const float arg = (base + gpref) - ex;
         if (arg < ex_cutoff) continue;
-        const double llc = L.llam0[l] - (double)vproj;
+        const double llc = llam0 - (double)vproj;
         const double pos = (llc - G.llam1) * G.inv_dllam;
         const int ic = lround_d(pos) + 1;
         const int f0 = ic < 1 ? 1 : (ic > NF ? NF : ic);
@@ -667,7 +672,7 @@ __global__ void __launch_bounds__(512, 1) k_opacity_adj(AtmosDev A, GridArgs G, 
         if (arg <= lref) continue;
         const float Rij = exp4(arg);
         if (voigt_peak * Rij <= refl) continue;
-        const float a = line_damping_a(L, l, unsold_c, lvb2, tothi, ne, starkpe) * G.sdl;
+        const float a = line_damping_a(line_damp(rec + l), unsold_c, lvb2, tothi, ne, starkpe) * G.sdl;
         const float S = Rij * qw.D;
         const float x1 = f0 == 1 ? (float)(-pos)
                                  : (float)(((f0 == NF ? llam_hi : G.llam[f0 - 1]) - llc) * G.inv_dllam);
@@ -698,10 +703,11 @@ __global__ void __launch_bounds__(512, 1) k_opacity_adj(AtmosDev A, GridArgs G, 
           deposit_adj_x2<NF, true, false>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
         else
           deposit_adj_x2<NF, false, false>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
-        // K is proportional to S = Rij D: dK/dD = K/D + dK/dih dih/dD
+        // K is proportional to S = Rij D: dK/dD = K/D + dK/dih dih/dD, the first term's
+        // sum over the lines from gB
         gB += Gl;
-        gE -= L.lower_ev[l] * Gl;
-        gD += Gl / qw.D + Hl * dih_dD(a, qw.D);
+        gE -= rec[l].lower_ev * Gl;
+        gD += Hl * dih_dD(a, qw.D);
         cg::coalesced_group grp = cg::coalesced_threads();
         const float tot = cg::reduce(grp, Gl, cg::plus<float>());
         if (grp.thread_rank() == 0) atomicAdd(&s_gp[sp * nline_max + l], tot);
@@ -710,7 +716,7 @@ __global__ void __launch_bounds__(512, 1) k_opacity_adj(AtmosDev A, GridArgs G, 
         const size_t o = (size_t)ncell * ((size_t)ray * A.nspecies + sp) + cs;
         p_lnbase[o] = gB;
         // D = sdl / idf
-        p_idf[o] = gD * (-qw.D / idf);
+        p_idf[o] = (gB / qw.D + gD) * (-qw.D / idf);
       }
     }
     if (live) p_ekt[rc] = gE;

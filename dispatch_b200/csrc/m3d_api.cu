@@ -383,6 +383,7 @@ void rot_planes(const double vec[3], const double ds_code[3], double bot2pivot, 
 LineArgs line_args(const m3d_linelist_t *ll) {
   LineArgs L;
   L.nline = ll->nline;
+  L.rec = nullptr;
   L.llam0 = ll->llam0;
   L.lower_ev = ll->lower_ev; L.gpref = ll->gpref; L.grad = ll->grad;
   L.gw1 = ll->gw1; L.gw2 = ll->gw2; L.gstk = ll->gstk;
@@ -1264,9 +1265,28 @@ int stage_synthesis(Staging &st, const m3d_atmos_t *atm, int nf, const double *n
       sp[k].L.nsel = in->d_nsel[k];
     }
   }
+  // the lines' records, which the FP32 lane kernels read
+  size_t nrec = 0;
+  int most = 0;
+  if (!fp64)
+    for (int k = 0; k < atm->nspecies; k++) {
+      nrec += (size_t)std::max(sp[k].L.nline, 0);
+      most = std::max(most, sp[k].L.nline);
+    }
+  if (nrec) {
+    void *rbuf;
+    TRY(scratch(39, sizeof(LineRec) * nrec, &rbuf));
+    LineRec *r = (LineRec *)rbuf;
+    for (int k = 0; k < atm->nspecies; k++) {
+      sp[k].L.rec = r;
+      r += std::max(sp[k].L.nline, 0);
+    }
+  }
   void *dsp;
   TRY(scratch(4, sizeof(SpeciesDev) * sp.size(), &dsp));
   CUDA_TRY(cudaMemcpyAsync(dsp, sp.data(), sizeof(SpeciesDev) * sp.size(), cudaMemcpyHostToDevice, g_ctx.stream));
+  if (nrec)
+    LAUNCH(k_line_records, dim3((most + 255) / 256, atm->nspecies), 256, 0, (const SpeciesDev *)dsp);
   A.species = (const SpeciesDev *)dsp;
   TRY(st.in(nu, nf, &in->dnu));
   TRY(st.in(llam, nf, &in->dllam));
@@ -1360,9 +1380,19 @@ int launch_opacity(SynthIn &in, const double *v, const double *d_vr, int nray, b
   using LaneKernel = void (*)(AtmosDev, GridArgs, const double *, float *, float *, const float2 *, const GridArgs *,
                               int, const double *, int, int, int *);
   LaneKernel k;
+  int threads = lane_threads(lf.NF);
+  const size_t cw = 32 / lf.P, units = (ncell * nray + cw - 1) / cw * in.nwin;
+  // No more units than 16 warps an SM: the units run side by side, once, and the SM waits
+  // on each warp's own chain of instructions, which 128 registers a thread shorten (a
+  // column of 80 points, 128 windows, 5 rays, 2000 lines: 2.80 -> 2.30 ms); above it
+  // the 24 warps of 80 registers win (96^3 cells with 20 warps of 96: 79 -> 84 ms).
+  const bool few = lf.NF == 32 && units <= (size_t)16 * sm_count();
+  if (few) threads = 512;
   if (lf.P > 1) k = k_lte_opacity_units_lane<64, false, false, false, false, true>;
+  else if (wins && few) k = k_lte_opacity_units_lane<32, false, false, true, false, false, 512>;
   else if (wins) k = k_lte_opacity_units_lane<32, false, false, true>;
   else if (nf == 32 && in.reach) k = k_lte_opacity_units_lane<32, true>;
+  else if (nf == 32 && few) k = k_lte_opacity_units_lane<32, false, false, false, false, false, 512>;
   else if (nf == 32) k = k_lte_opacity_units_lane<32, false>;
   else if (lf.NF == 16) k = k_lte_opacity_units_lane<16, false, false, false, true>;
   else if (lf.NF == 32) k = k_lte_opacity_units_lane<32, false, false, false, true>;
@@ -1371,9 +1401,8 @@ int launch_opacity(SynthIn &in, const double *v, const double *d_vr, int nray, b
   TRY(lane_attr((const void *)k));
   int *next;
   TRY(unit_counter(&next));
-  const size_t cw = 32 / lf.P, units = (ncell * nray + cw - 1) / cw * in.nwin;
   const int grid = (int)std::min<size_t>(units, (size_t)sm_count());
-  LAUNCH_S(M3D_STAGE_OPACITY, k, grid, lane_threads(lf.NF), 2 * QLG_NTAB * sizeof(float), in.A, in.G, in.dnu,
+  LAUNCH_S(M3D_STAGE_OPACITY, k, grid, threads, 2 * QLG_NTAB * sizeof(float), in.A, in.G, in.dnu,
            (float *)dchi, (float *)dS, g_ctx.d_tab, in.d_Gw, in.nwin, d_vr, nray, lf.P, next);
   return M3D_OK;
 }

@@ -77,8 +77,24 @@ __global__ void k_qlg_profile(int n, const float2 *tab, const float *a, const fl
 // ----------------------------------------------------------------------------
 // Line opacity of one cell by one warp (add_opacity_equi, linelist_mod.f90:729-960)
 // ----------------------------------------------------------------------------
+// One line of the lane kernels' loops, two 16-byte loads: every lane of a warp reads the
+// same line, and eight loads from eight arrays, their pointers loaded first, took a
+// tenth of the loop's instructions and their latency besides (96^3 cells, 500 lines, 13
+// rays: 91.5 -> 79 ms; reading the next line's record ahead gave no more).  Built for
+// each call by k_line_records.  Two marks
+// share slots that mean nothing beside them: gpref holds LINE_OFF for a line that is not
+// active, gw2 holds LINE_UNSOLD for one with the Unsold law (a list's own NaN there is
+// stored as 0x7fc00000).
+struct alignas(16) LineRec {
+  double llam0;
+  float lower_ev, gpref;
+  float grad, gw1, gw2, gstk;
+};
+constexpr uint32_t LINE_OFF = 0x7fd0ff01u, LINE_UNSOLD = 0x7fd0ff02u;
+
 struct LineArgs {
   int nline;
+  const LineRec *rec;
   const double *llam0;
   const float *lower_ev, *gpref, *grad, *gw1, *gw2, *gstk;
   const uint8_t *unsold;
@@ -114,6 +130,26 @@ __device__ __forceinline__ float line_damping_a(const LineArgs &L, int l, float 
   else a = fmaf(-gs, starkpe, a);
   return a;
 }
+
+// the same from the line's record
+__device__ __forceinline__ float line_damping_a(const float4 &q, float unsold_c, float lvb2, float tothi, float ne,
+                                                float starkpe) {
+  float a = q.x;
+  if (__float_as_uint(q.z) == LINE_UNSOLD) a = fmaf(q.y, unsold_c, a);
+  else if (q.y != 0.0f) a = fmaf(q.y * exp4(q.z * lvb2), tothi, a);
+  if (q.w >= 0.0f) a = fmaf(q.w, ne, a);
+  else a = fmaf(-q.w, starkpe, a);
+  return a;
+}
+
+// a record's halves: the place and strength of the line, its damping
+__device__ __forceinline__ void line_place(const LineRec *r, double &llam0, float &lower_ev, float &gpref) {
+  const uint4 q = __ldg(reinterpret_cast<const uint4 *>(r));
+  llam0 = __hiloint2double((int)q.y, (int)q.x);
+  lower_ev = __uint_as_float(q.z);
+  gpref = __uint_as_float(q.w);
+}
+__device__ __forceinline__ float4 line_damp(const LineRec *r) { return __ldg(reinterpret_cast<const float4 *>(r) + 1); }
 
 // chi, eta, cont, logref point at this cell's nf values (shared or global memory).
 // dep(level) returns the departure coefficient of a 1-based level of this cell.

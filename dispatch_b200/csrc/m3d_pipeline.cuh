@@ -27,6 +27,24 @@ struct AtmosDev {
   float maser_chi_floor;
 };
 
+// The records of every species' lines: species along the grid's second dimension
+__global__ void k_line_records(const SpeciesDev *species) {
+  const LineArgs &L = species[blockIdx.y].L;
+  LineRec *rec = const_cast<LineRec *>(L.rec);
+  for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < L.nline; l += gridDim.x * blockDim.x) {
+    auto plain = [](float x) { return x != x ? __uint_as_float(0x7fc00000u) : x; };
+    LineRec r;
+    r.llam0 = L.llam0[l];
+    r.lower_ev = L.lower_ev[l];
+    r.gpref = L.active && !L.active[l] ? __uint_as_float(LINE_OFF) : plain(L.gpref[l]);
+    r.grad = L.grad[l];
+    r.gw1 = L.gw1[l];
+    r.gw2 = L.unsold[l] ? __uint_as_float(LINE_UNSOLD) : plain(L.gw2[l]);
+    r.gstk = L.gstk[l];
+    rec[l] = r;
+  }
+}
+
 // Work units and transfer units of one point, FP32 (rt_patch_mod.f90:2004-2023,
 // 2309-2326, 3518-3536, 3571-3651, composition_mod.f90:1848-1858)
 __device__ __forceinline__ void point_units(float chi_c, float h_kT, double nu, float chil, float etal, float fl,
@@ -331,8 +349,9 @@ __host__ __device__ constexpr int lane_threads(int NF) { return NF <= 16 ? 1024 
 // from a counter (*next, zero at the launch): a unit's time follows its cells' lines,
 // and warps that strode over a fixed share of the units left the 96^3 cube 4 % slower
 // than blocks handed out by the hardware.
-template <int NF, bool REACH, bool CHIL = false, bool WINS = false, bool PAD = false, bool MULTI = false>
-__global__ void __launch_bounds__(lane_threads(NF), 1)
+template <int NF, bool REACH, bool CHIL = false, bool WINS = false, bool PAD = false, bool MULTI = false,
+          int TH = lane_threads(NF)>
+__global__ void __launch_bounds__(TH, 1)
     k_lte_opacity_units_lane(AtmosDev A, GridArgs G0, const double *nu0, float *chi_out, float *S_out,
                              const float2 *tab, const GridArgs *Gw, int nwin, const double *vr, int nray, int P_,
                              int *next) {
@@ -388,14 +407,18 @@ __global__ void __launch_bounds__(lane_threads(NF), 1)
       const QlgCell qw = qlg_cell(G.sdl / idf);
       const float lvb2 = logf_m3d(Sd.vbar2[cs]);
       const float unsold_c = exp4(0.3f * lvb2) * tothi;
+      const LineRec *rec = L.rec;
       const int nline = REACH ? *L.nsel : L.nline;
       for (int s = 0; s < nline; s++) {
         const int l = REACH ? L.sel[s] : s;
-        if (L.active && !L.active[l]) continue;
-        const float ex = L.lower_ev[l] * ekt;
-        const float arg = (base + L.gpref[l]) - ex;
+        double llam0;
+        float lower_ev, gpref;
+        line_place(rec + l, llam0, lower_ev, gpref);
+        if (__float_as_uint(gpref) == LINE_OFF) continue;
+        const float ex = lower_ev * ekt;
+        const float arg = (base + gpref) - ex;
         if (arg < ex_cutoff) continue;
-        const double llc = L.llam0[l] - (double)vproj;
+        const double llc = llam0 - (double)vproj;
         const double pos = (llc - G.llam1) * G.inv_dllam;
         const int ic = lround_d(pos) + 1;
         const int f0 = ic < 1 ? 1 : (ic > nf ? nf : ic);
@@ -428,7 +451,7 @@ __global__ void __launch_bounds__(lane_threads(NF), 1)
         }
         const float Rij = exp4(arg);
         if (!outside && voigt_peak * Rij <= refl) continue;
-        const float a = line_damping_a(L, l, unsold_c, lvb2, tothi, ne, starkpe) * G.sdl;
+        const float a = line_damping_a(line_damp(rec + l), unsold_c, lvb2, tothi, ne, starkpe) * G.sdl;
         const float S = Rij * qw.D;
         // (llam(f0) - llc)/dllam; at f0 = 1 it is -pos exactly (the rounded difference
         // and product are odd in their sign)
