@@ -586,6 +586,11 @@ __device__ __forceinline__ void deposit_adj_x2(float (&chl)[NF], const float (&g
 // share the launch, the warps fetching their units as in the forward kernel; a ray's
 // per-cell sums go to its own part (p_*, ray after ray), which k_add_rays adds in the
 // rays' order, so that these gradients do not depend on the launch.
+// Bound by issue, with the 32 registers each of chi_l and its adjoint: 128 registers, 16
+// warps an SM (blocks of 384 and 256 threads with more: no faster).  32 x 32 x 64 cells,
+// ten species of 100 lines, forward and backward: 78.7 ms with one ray a launch and one
+// point an instruction, 43.8 with rays together and pairs of points, 38 with the line
+// records.
 // Shared memory: the QLG tables (float2), the table differences dW, and the block's
 // per-line sums (nline floats).
 __global__ void __launch_bounds__(512, 1) k_opacity_adj(AtmosDev A, GridArgs G, const double *nu, const double *vr,

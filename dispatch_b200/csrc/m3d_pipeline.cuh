@@ -1,9 +1,11 @@
 // The LTE synthesis output pass (rt_patch_t%execute do_final branch,
 // rt_patch_mod.f90:1014-1030) as two kernels per ray direction:
 //
-//   k_lte_opacity_units  warp per cell: LTE background (beta, Bnu), work units
-//                        (xhat, ehat), logref, the line opacity of every species in
-//                        line order, and work_to_transfer_units -> (chi, Snu)
+//   k_lte_opacity_units_lane  lane per (ray, cell): LTE background (beta, Bnu), work
+//                        units (xhat, ehat), logref, the line opacity of every species
+//                        in line order, and work_to_transfer_units -> (chi, Snu);
+//                        k_lte_opacity_units (warp per cell) for the windows and lists
+//                        it does not take, k_lte_opacity_units_f64 in double
 //   k_quad_rot_column    thread per (f, x, y): the whole column bottom to top, slab
 //                        by slab, with rotate_array fused into the loads, the
 //                        PCHIP ghost below the bottom slab, long_char_quadratic,
@@ -325,7 +327,8 @@ __device__ __forceinline__ float pick(const float (&a)[NF], int i) {
 
 // Threads of the lane kernel's block, one block per SM: as many warps as the NF
 // registers of chi_l and the line's working set leave room for (64, 80, 96 and 128
-// registers a thread)
+// registers a thread).  At 32 frequencies 28 warps of 72 registers spill (96^3 cells:
+// 84.5 ms against 79.9) and 20 of 96 issue less (84.2)
 __host__ __device__ constexpr int lane_threads(int NF) { return NF <= 16 ? 1024 : NF <= 32 ? 768 : NF <= 48 ? 640 : 512; }
 
 // REACH: the line list carries reach_in (has_reach): the lines select_lines kept,

@@ -25,8 +25,8 @@ constexpr int SE_NMAX = 64;
 constexpr int SE_COL_REGEMORTER = 1, SE_COL_SEATON = 2;
 constexpr int SE_COLH_DRAWIN = 1, SE_COLH_TAKEDA = 2;
 
-// A bound pair under van Regemorter's recipe: its energy, f/dev, 1-in-16-bytes beside
-// its levels
+// A bound pair under van Regemorter's recipe: its energy, f/dev and the
+// weight g_i beside its levels, two 16-byte loads
 struct __align__(16) SePair { double dev, fdev; int i, j; double gi; };
 
 // Atom tables in device memory.  Transitions are listed by round: the
@@ -452,9 +452,10 @@ __device__ __forceinline__ void se_solve_no_pivot(double *W, double *e, int n, i
 // move one place down.  Row k is final at step k; its thread writes it to shared memory
 // (U, rows of LD doubles, element j of row k at column k + j), where every other row
 // reads it back by broadcast, two elements a load.  The rows shrink by eight registers
-// every eight steps.  Where the start kept the matrix in shared memory, each update
-// cost two shared loads and a store (88 % of the 21-level update's 8.2 ms a 262144
-// cells, and 5 to 7 cells an SM at 61 levels).
+// every eight steps.  With the matrix in shared memory each update cost two shared loads
+// and a store, 88 % of the 21-level update's time, and 5 to 7 cells fitted an SM at 61
+// levels.  262144 cells of 21 levels: 8.80 -> 3.72 ms with the collision pairs' records;
+// 40000 of 61: 9.14 -> 5.12 ms.
 //
 // A row whose pivot element vanishes is updated like the others, where the
 // shared-memory form skips it: a - l 0 is a for every finite l (but for the sign of a
@@ -697,7 +698,9 @@ __host__ __device__ inline size_t se_team_doubles(int n, int N) {
 }
 
 // blocks per SM that the register form's rows leave room for: its N doubles a thread
-// and some fifty registers beside them; the general collision forms take what they need
+// and some fifty registers beside them; the general collision forms take what they need.
+// 21 levels, 262144 cells: 4.27 ms at 4 blocks, 3.82 at 5, 3.71 at 6, 3.81 at 7; 61
+// levels, 40000 cells: 6.77 at 4 (255 registers), 5.12 at 5 and 6.
 __host__ __device__ constexpr int se_threads(int TEAM, int N) { return N == 0 ? 128 : TEAM == 64 ? 64 : 128; }
 __host__ __device__ constexpr int se_min_blocks(int CM, int N) {
   return N == 0 ? (CM == 2 ? 2 : 4) : CM == 2 ? 1 : N <= 24 ? 6 : N <= 32 ? 4 : N <= 48 ? 7 : 6;
