@@ -275,12 +275,13 @@ __global__ void __launch_bounds__(32 * kOptabWarps, 2) k_optab_sample_ll(OptabDe
       for (int g = 0; g < G; g++) {
         if (g >= ncl) break;
         const double x = __dmul_rn(lq, cells[wib][g].vf);
-        while (lhi < x) {
+        // bounded by the count: an infinite x passes no comparison with the ends' marks
+        while (cnt < nnu && lhi < x) {
           cnt++;
           llo = lhi;
           lhi = cnt < nnu ? lam[cnt] : HUGE_VAL;
         }
-        while (llo >= x) {
+        while (cnt > 0 && llo >= x) {
           cnt--;
           lhi = llo;
           llo = cnt > 0 ? lam[cnt - 1] : -HUGE_VAL;
