@@ -533,9 +533,9 @@ __device__ __forceinline__ void se_solve_rows(const double *W, int ldw, double *
 #pragma unroll 8
       for (int j = 2; j < n - i; j++) t = t - u[j];
       x = t / u[0];
-      if (row == 0) es[i] = x;
       for (int r = row; r <= i - 2; r += 32) U[LD * r + i - r] = U[LD * r + i - r] * x;
       __syncwarp();
+      if (row == 0) es[i] = x;   // every lane has read the right-hand side there
     }
   }
   team_sync<TEAM>();
