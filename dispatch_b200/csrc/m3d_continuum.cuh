@@ -9,8 +9,8 @@
 //   electron_scattering, rayleigh_scattering   :3851-3939
 //   'H BF' under occupation probabilities: wcalc2   level_mod.f90:149-279 (its
 //                                    per-wavelength set-up, calc_x_and_k :77-94, on the host)
-// One warp per cell: the lanes first form each component's temperature stencil and
-// absorption factor for the cell (one component per lane), then run along the
+// A warp per cell, or per four: the lanes first form each component's temperature stencil
+// and absorption factor for the cells (one component per lane), then run along the
 // window's wavelengths, each adding the components in their order.  Kinds follow the
 // Fortran: tables, xhat and sigma real(4); the EOS state, the absorption factors and
 // the wavelength cubes real(8); a real(4) value updated from a real(8) expression is
@@ -20,12 +20,9 @@
 
 namespace m3d {
 
-constexpr int kContWarps = 8;     // warps per block
-constexpr int kContCells = 4;     // cells a warp works on at a time
 constexpr int kContMaxComp = 64;  // components of one call
 constexpr int kContMaxRows = 1024;  // table rows a window reads, over all components (per cell, in shared memory)
 constexpr int kContMaxTab = 8192;   // their table entries at every temperature node (per block, in shared memory)
-constexpr int kContKF = 1;          // wavelengths a lane holds of each cell in one pass over the components
 
 // wcalc2's per-wavelength set-up of an 'H BF' level (level_mod.f90:186-218): cls 0
 // none, 1 beyond the series limit, 2 below it (a dissolved upper level); qcut =
@@ -391,32 +388,44 @@ __global__ void k_continuum_lam(int nlam, const double *__restrict__ lam, int he
 // The per-cell scalars of the wavelength loop, in shared memory
 struct ContCellLoc { double hrest, hk_T, nHI, nHe, nH2, els; };
 
-// shared memory beside the components' descriptors, the staged table entries and each
-// warp's rows: per warp and cell the scalars and the components' states
-__host__ __device__ inline size_t cont_cell_bytes(int ncomp) {
-  return kContWarps * kContCells * (sizeof(ContCellLoc) + sizeof(BfCellDev) * (size_t)ncomp);
+// dynamic shared memory of a block of W warps with C cells each: the components'
+// descriptors, per cell its scalars and its components' states, the staged table entries,
+// and each cell's rows
+__host__ __device__ inline size_t cont_cell_bytes(int ncomp, int cells) {
+  return cells * (sizeof(ContCellLoc) + sizeof(BfCellDev) * (size_t)ncomp);
+}
+__host__ __device__ inline size_t cont_smem(int ncomp, int cells, int rows_used, int tab_used) {
+  return sizeof(BfCompDev) * (size_t)ncomp + cont_cell_bytes(ncomp, cells) +
+         sizeof(float) * ((size_t)tab_used + (size_t)cells * rows_used);
 }
 
-// A warp takes four neighbouring cells: their components' temperature stencils and factors
-// side by side in its lanes, their rows in one pass, and each wavelength's stencil,
-// Gaunt-like table value and Rayleigh terms read once for all.  64 registers at four
-// blocks of eight warps per SM, so the window's table rows are staged four times an SM
-// instead of eight and L1 keeps the stencils.  262144 cells, 250 wavelengths, fourteen
-// components: 3.76 -> 2.49 ms against a cell a warp with eight wavelengths a lane (two
-// cells and two wavelengths 2.66, three and two 2.55, four and two 3.08 with spills, six
-// and one 2.74).
-__global__ void __launch_bounds__(kContWarps * 32, 4)
+// W warps a block, C neighbouring cells a warp, KF wavelengths of each a lane and pass.
+//
+// <8, 4, 1, 4>: the cells' temperature stencils and factors side by side in the lanes,
+// their rows in one pass, and each wavelength's stencil, Gaunt-like table value and
+// Rayleigh terms read once for all.  64 registers at four blocks per SM, so the window's
+// table rows are staged four times an SM and L1 keeps the stencils.
+// 262144 cells, 250 wavelengths, fourteen components: 3.76 -> 2.49 ms against a cell a
+// warp with eight wavelengths a lane (two cells and two wavelengths 2.66, three and two
+// 2.55, four and two 3.08 with spills, six and one 2.74).
+//
+// <8, 1, 4, 4>: a cell a warp with four wavelengths a lane, for the calls whose cells are
+// too few for the other form's warps or whose rows, 128 bytes each there and 32 here, leave
+// it less than three blocks an SM.  64 registers, 24 bytes spilled; against one block of
+// four warps with eight wavelengths a lane, two wavelengths and three: 2000 cells 317 us
+// (333, 326, 325), 110592 cells and 28 components 3.06 ms (4.45, 3.45, 3.25).
+template <int W, int C, int KF, int MINB>
+__global__ void __launch_bounds__(W * 32, MINB)
 k_continuum(int ncomp, const BfCompDev *__restrict__ comps_g, int any_istim, int nlam, ContLamDev LW,
             const double *__restrict__ nu, int ncell, ContCellsDev S, const float *__restrict__ beta,
             float *__restrict__ xhat, float *__restrict__ sigma, int rows_used, int tab_used) {
-  constexpr int C = kContCells;
   extern __shared__ __align__(16) float cont_sh[];
   BfCompDev *scomp = reinterpret_cast<BfCompDev *>(cont_sh);   // (ncomp) the components' descriptors
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   ContCellLoc *loc = reinterpret_cast<ContCellLoc *>(scomp + ncomp) + wib * C;
-  BfCellDev *st = reinterpret_cast<BfCellDev *>(reinterpret_cast<ContCellLoc *>(scomp + ncomp) + kContWarps * C) +
+  BfCellDev *st = reinterpret_cast<BfCellDev *>(reinterpret_cast<ContCellLoc *>(scomp + ncomp) + W * C) +
                   (size_t)wib * C * ncomp;
-  float *stab = reinterpret_cast<float *>(reinterpret_cast<char *>(scomp + ncomp) + cont_cell_bytes(ncomp));
+  float *stab = reinterpret_cast<float *>(reinterpret_cast<char *>(scomp + ncomp) + cont_cell_bytes(ncomp, W * C));
   float *rows = stab + tab_used + (size_t)wib * C * rows_used;   // (C, rows_used) the cells' rows
   {
     const int nw = ncomp * (int)(sizeof(BfCompDev) / sizeof(int));
@@ -437,9 +446,9 @@ k_continuum(int ncomp, const BfCompDev *__restrict__ comps_g, int any_istim, int
     }
   }
   __syncthreads();
-  const int nwarp = gridDim.x * kContWarps;
+  const int nwarp = gridDim.x * W;
   const double thomson = cont_thomson();
-  for (int x0 = (blockIdx.x * kContWarps + wib) * C; x0 < ncell; x0 += nwarp * C) {
+  for (int x0 = (blockIdx.x * W + wib) * C; x0 < ncell; x0 += nwarp * C) {
     // a last cell without a neighbour is worked on twice and written once
     int x[C];
 #pragma unroll
@@ -507,10 +516,10 @@ k_continuum(int ncomp, const BfCompDev *__restrict__ comps_g, int any_istim, int
       }
     }
     __syncwarp();
-    for (int f0 = lane; f0 - lane < nlam; f0 += 32 * kContKF) {
-      float v[C][kContKF];
+    for (int f0 = lane; f0 - lane < nlam; f0 += 32 * KF) {
+      float v[C][KF];
 #pragma unroll
-      for (int k = 0; k < kContKF; k++) {
+      for (int k = 0; k < KF; k++) {
         const int f = f0 + 32 * k;
         const double c3 = f < nlam ? __ldg(LW.cube + f) : 0.0;
 #pragma unroll
@@ -518,20 +527,20 @@ k_continuum(int ncomp, const BfCompDev *__restrict__ comps_g, int any_istim, int
       }
       for (int j = 0; j < ncomp; j++) {
         const BfCompDev &c = comps[j];
-        if (!c.istim) cont_comp<kContKF, C>(c, st + j, ncomp, rows, rows_used, f0, LW.l3, S, x, v);
+        if (!c.istim) cont_comp<KF, C>(c, st + j, ncomp, rows, rows_used, f0, LW.l3, S, x, v);
       }
       if (any_istim) {
-        float tmp[C][kContKF];
+        float tmp[C][KF];
 #pragma unroll
         for (int q = 0; q < C; q++)
 #pragma unroll
-          for (int k = 0; k < kContKF; k++) tmp[q][k] = 0.0f;
+          for (int k = 0; k < KF; k++) tmp[q][k] = 0.0f;
         for (int j = 0; j < ncomp; j++) {
           const BfCompDev &c = comps[j];
-          if (c.istim) cont_comp<kContKF, C>(c, st + j, ncomp, rows, rows_used, f0, LW.l3, S, x, tmp);
+          if (c.istim) cont_comp<KF, C>(c, st + j, ncomp, rows, rows_used, f0, LW.l3, S, x, tmp);
         }
 #pragma unroll
-        for (int k = 0; k < kContKF; k++) {
+        for (int k = 0; k < KF; k++) {
           const int f = f0 + 32 * k;
           if (f >= nlam) break;
 #pragma unroll
@@ -548,7 +557,7 @@ k_continuum(int ncomp, const BfCompDev *__restrict__ comps_g, int any_istim, int
         }
       }
 #pragma unroll
-      for (int k = 0; k < kContKF; k++) {
+      for (int k = 0; k < KF; k++) {
         const int f = f0 + 32 * k;
         if (f >= nlam) break;
         const double xr = sigma ? __ldg(LW.xr + f) : 0.0, rh = sigma ? __ldg(LW.rayh + f) : 0.0;
