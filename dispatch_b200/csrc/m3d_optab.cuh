@@ -327,6 +327,104 @@ __global__ void __launch_bounds__(32 * kOptabWarps, 2) k_optab_sample_ll(OptabDe
   }
 }
 
+// ---- a cell a warp ----------------------------------------------------------------
+// For cell counts that give the grouped kernels less than the warps they need: the
+// neighbours' turns in a warp then only add up.  64 registers at 4 blocks an SM, the
+// corners read pair by pair.  The cells are called small below a full round of the
+// grouped kernel's warps on the GPU (28416 cells), for the line list below six (56832),
+// whose last round of longer turns weighs more.  256 frequencies, a cell a warp against
+// groups: 512 cells 44 and 58 us, for the line list 79 and 95; 4096 cells 41 / 48 and
+// 69 / 83; 13824 57 / 56 and 106 / 118; 32768 86 / 78 and 196 / 203; 64000 140 / 108 and
+// 345 / 325.
+
+// collapse of a query between the nodes at and at + 1
+__device__ __forceinline__ float optab_collapse_at(const float4 *t, long long at, int sit, long long sje,
+                                                   const float w[5], const float4 tc, const float4 nc) {
+  float v[4], gt[4], ge[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const long long a = at + (c & 1) * sit + (c >> 1) * sje;
+    const float4 A = __ldg(t + a), B = __ldg(t + a + 1);
+    v[c] = fmaf(w[4], B.y, fmaf(w[3], A.y, fmaf(w[2], B.x, w[1] * A.x)));
+    gt[c] = fmaf(w[0], B.z, w[1] * A.z);
+    ge[c] = fmaf(w[0], B.w, w[1] * A.w);
+  }
+  return optab_collapse_pc(v, gt, ge, tc, nc);
+}
+
+// and of one on the node at
+__device__ __forceinline__ float optab_collapse_node_at(const float4 *t, long long at, int sit, long long sje,
+                                                        const float4 tc, const float4 nc) {
+  float4 A[4];
+  optab_corners(t, at, sit, sje, A);
+  return optab_collapse_node(A, tc, nc);
+}
+
+__global__ void __launch_bounds__(32 * kOptabWarps, 4) k_optab_sample_one(OptabDev T, int nf, long long ncell,
+                                                                       const double *temp, const double *ne,
+                                                                       const float *chi500, const OptabFreq *fc,
+                                                                       float *back, float *scat) {
+  const int lane = threadIdx.x & 31;
+  const long long w0 = (long long)blockIdx.x * kOptabWarps + (threadIdx.x >> 5);
+  const long long nw = (long long)gridDim.x * kOptabWarps;
+  const int sit = T.nnu;
+  const long long sje = (long long)T.nnu * T.ntemp;
+  for (long long c = w0; c < ncell; c += nw) {
+    const OptabCell q = optab_cell_of(T, temp[c], ne[c], chi500[c], 1.0);
+    for (int f = lane; f < nf; f += 32) {
+      const OptabFreq p = fc[f];
+      float kap, kas;
+      if (p.node >= 0) {
+        kap = optab_collapse_node_at(T.tv, q.base + p.node, sit, sje, q.tc, q.nc);
+        kas = optab_collapse_node_at(T.ts, q.base + p.node, sit, sje, q.tc, q.nc);
+      } else {
+        const float w[5] = {p.pl, p.wc0, p.wc1, p.wcm0, p.wcm1};
+        kap = optab_collapse_at(T.tv, q.base + p.k, sit, sje, w, q.tc, q.nc);
+        kas = optab_collapse_at(T.ts, q.base + p.k, sit, sje, w, q.tc, q.nc);
+      }
+      const size_t o = (size_t)c * nf + f;
+      back[o] = (kap + kas) * q.ch;
+      scat[o] = kas * q.ch;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(32 * kOptabWarps, 4) k_optab_sample_ll_one(OptabDev T, int nf, long long ncell,
+                                                                          const double *temp, const double *ne,
+                                                                          const float *chi500, const float *vproj,
+                                                                          const double *lam_q, const OptabFreq *fc,
+                                                                          float *xhat, float *ehat,
+                                                                          float *chi_scat) {
+  const int lane = threadIdx.x & 31;
+  const long long w0 = (long long)blockIdx.x * kOptabWarps + (threadIdx.x >> 5);
+  const long long nw = (long long)gridDim.x * kOptabWarps;
+  const int sit = T.nnu, nnu = T.nnu;
+  const long long sje = (long long)T.nnu * T.ntemp;
+  const double *lam = T.lam;
+  for (long long c = w0; c < ncell; c += nw) {
+    const OptabCell q = optab_cell_of(T, temp[c], ne[c], chi500[c], 1.0 + (double)vproj[c]);
+    for (int f = lane; f < nf; f += 32) {
+      // the work slots before the bracket and the table
+      const size_t o = (size_t)c * nf + f;
+      const float xv = xhat[o], ev = ehat[o], sv = chi_scat ? chi_scat[o] : 0.0f;
+      const double x = __dmul_rn(lam_q[f], q.vf);
+      int cnt = fc[f].cnt;
+      while (cnt < nnu && lam[cnt] < x) cnt++;
+      while (cnt > 0 && lam[cnt - 1] >= x) cnt--;
+      float w[5];
+      const int k = optab_interval(nnu, lam, cnt, x, w), nd = optab_on_node(w, k);
+      auto kappa = [&](const float4 *t) {
+        return nd >= 0 ? optab_collapse_node_at(t, q.base + nd, sit, sje, q.tc, q.nc)
+                       : optab_collapse_at(t, q.base + k, sit, sje, w, q.tc, q.nc);
+      };
+      const float add = kappa(T.tv) * q.ch;
+      xhat[o] = xv + add;
+      ehat[o] = ev + add;
+      if (chi_scat) chi_scat[o] = sv + kappa(T.ts) * q.ch;
+    }
+  }
+}
+
 // sample_build_derivatives (optab_mod.f90:125-166), one thread per node.
 // pchip_slopes8 (interpol_mod.f90:240-284) along the fp64 wavelength nodes:
 // the interior slope of node i of a line y (stride 1)

@@ -1,15 +1,18 @@
-"""Cell counts on both sides of the line that parts the one-cell and the grouped form of
-the continuum, groups left short among them, and windows of many table rows: bit for bit
-against the oracle."""
+"""Cell counts on both sides of the lines that part the one-cell and the grouped forms of
+the continuum and of the table samplers, groups left short among them: bit for bit
+against the oracle.  Below the lines the grouped forms, which the small counts of other
+tests no longer reach, are not taken."""
 import numpy as np
 import pytest
 
+import optab_cases as ocases
 from dispatch_b200 import synth
 
 pytestmark = pytest.mark.gpu
 
 SMS = 148
 CONT = SMS * 64                  # the continuum's line
+BG, LL = SMS * 3 * 8 * 8, SMS * 2 * 8 * 4 * 6
 
 
 def _exact_comps(comps):
@@ -57,3 +60,28 @@ def test_continuum_table_rows(m3d, oracle, ncell, nnu, ncomp):
     base = [_refined(c, nnu) for c in _exact_comps(comps)]
     comps = (base * (ncomp // len(base) + 1))[:ncomp]
     _continuum(comps, lam, nu, cells, ncell)
+
+
+@pytest.mark.parametrize("ncell", [BG - 1, BG, BG + 1, BG + 7, LL - 1, LL, LL + 1, LL + 3])
+def test_table_counts(m3d, oracle, ncell):
+    from dispatch_b200.optab import SampleOptab
+    from oracle import optab
+    c = ocases.cells(seed=3, nx=40, ny=40, nz=36)
+    tab = ocases.table("linelist", nnu=120, cells_=c)
+    c = {k: np.ascontiguousarray(v[:ncell]) for k, v in c.items()}
+    assert c["temp"].size == ncell
+    q = np.sort(np.concatenate([tab["lam"][20:60:10], np.linspace(3900.0, 9100.0, 29)]))
+    T = SampleOptab.from_dict(tab)
+    for g, o in zip(T.interpolate(c["temp"], c["ne"], c["chi500"], q),
+                    optab.sample(tab, c["temp"], c["ne"], c["chi500"], q)):
+        np.testing.assert_array_equal(g, o)
+    vp = (c["vproj"] * 40.0).astype(np.float32)
+    vp[::97] = np.float32(-np.inf)
+    rng = np.random.default_rng(5)
+    base = [rng.random((ncell, q.size)).astype(np.float32) for _ in range(3)]
+    gpu, ref = [b.copy() for b in base], [b.copy() for b in base]
+    T.interpolate_ll(c["temp"], c["ne"], c["chi500"], gpu[0], gpu[1], q, vp, chi_scat=gpu[2])
+    optab.sample_ll(tab, c["temp"], c["ne"], c["chi500"], vp, q, ref[0], ref[1], ref[2])
+    for g, o in zip(gpu, ref):
+        np.testing.assert_array_equal(g, o)
+    T.close()
