@@ -1323,8 +1323,8 @@ int rays_per_launch(size_t ncell, int nf, int nray, size_t esz) {
 // Line opacity + transfer units of every cell for nray directions (d_vr on the device,
 // v their host copy): (chi, S) of the window, frequency fastest per cell, ray after ray.
 // FP32: the lane-per-cell kernel; the warp-per-cell kernel for windows below 8
-// frequencies, and for lists with reach_in unless the window has 32 (one ray a launch
-// either way).  FP64: the plain FP64 kernel.
+// frequencies, for one ray of a small atmosphere, and for lists with reach_in unless the
+// window has 32 frequencies (one ray a launch each).  FP64: the plain FP64 kernel.
 int launch_opacity(SynthIn &in, const double *v, const double *d_vr, int nray, bool fp64, void *dchi, void *dS) {
   const int nf = in.nf;
   const size_t ncell = in.ncell;
@@ -1359,7 +1359,14 @@ int launch_opacity(SynthIn &in, const double *v, const double *d_vr, int nray, b
              in.d_nsel[k]);
   }
   const LaneForm lf = lane_form(nf);
-  if (lf.NF == 0 || (in.reach && nf != 32)) {
+  // One ray of no more cells than one round of the warp-per-cell kernel's warps (16 an SM
+  // beside its tables): each warp then runs one cell's lines, a lane a frequency, where
+  // the lane kernel's few warps run 32 cells' one frequency after the other.  500 lines,
+  // by the warp and by the lane kernel: 80 cells x 20 frequencies 594 / 728 us, x 64 645 /
+  // 922; 1024 cells x 45 620 / 772; 2000 x 100 769 / 947; 2940 x 45 842 / 791; 80 x 256
+  // 1017 / 1016.  (32 frequencies: 780 / 612, by the lane kernel's form of few units.)
+  const bool lone = nray == 1 && nf != 32 && nf <= 128 && ncell <= (size_t)16 * sm_count();
+  if (lf.NF == 0 || lone || (in.reach && nf != 32)) {
     const size_t smem = (2 * QLG_NTAB + (size_t)warps * 4 * nf) * sizeof(float);
     thread_local size_t attr = 0;
     if (attr < smem) {
@@ -1386,13 +1393,13 @@ int launch_opacity(SynthIn &in, const double *v, const double *d_vr, int nray, b
   // on each warp's own chain of instructions, which 128 registers a thread shorten (a
   // column of 80 points, 128 windows, 5 rays, 2000 lines: 2.80 -> 2.30 ms); above it
   // the 24 warps of 80 registers win (96^3 cells with 20 warps of 96: 79 -> 84 ms).
-  const bool few = lf.NF == 32 && units <= (size_t)16 * sm_count();
+  const bool few = nf == 32 && !in.reach && units <= (size_t)16 * sm_count();
   if (few) threads = 512;
   if (lf.P > 1) k = k_lte_opacity_units_lane<64, false, false, false, false, true>;
   else if (wins && few) k = k_lte_opacity_units_lane<32, false, false, true, false, false, 512>;
   else if (wins) k = k_lte_opacity_units_lane<32, false, false, true>;
   else if (nf == 32 && in.reach) k = k_lte_opacity_units_lane<32, true>;
-  else if (nf == 32 && few) k = k_lte_opacity_units_lane<32, false, false, false, false, false, 512>;
+  else if (few) k = k_lte_opacity_units_lane<32, false, false, false, false, false, 512>;
   else if (nf == 32) k = k_lte_opacity_units_lane<32, false>;
   else if (lf.NF == 16) k = k_lte_opacity_units_lane<16, false, false, false, true>;
   else if (lf.NF == 32) k = k_lte_opacity_units_lane<32, false, false, false, true>;
