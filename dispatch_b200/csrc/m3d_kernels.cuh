@@ -166,7 +166,7 @@ __device__ void warp_cell_lines(const LineArgs &L, const GridArgs &G, const Cell
   const float ex_cutoff = -85.0f, voigt_peak = 0.5641895835f, sqrt_pi = 1.7724538509f;
   const int nf = G.nf;
   const QlgCell qw = qlg_cell(G.sdl / c.idf);
-  const float lvb2 = logf_m3d(c.vbar2);
+  const float lvb2 = logf_m3d<true>(c.vbar2);
   const float unsold_c = exp4(0.3f * lvb2) * c.tothi;
   const int nline = L.sel ? *L.nsel : L.nline;
   const double lam_lo = G.llam[0], lam_hi = G.llam[nf - 1];
@@ -224,7 +224,7 @@ __device__ void warp_cell_lines(const LineArgs &L, const GridArgs &G, const Cell
       } else {
         refl = G.tol * cont[f0 - 1];
         const float flo = G.flo_scale * chi[f0 - 1];
-        if (flo > refl) { refl = flo; lref = logf_m3d(flo * sqrt_pi); }
+        if (flo > refl) { refl = flo; lref = logf_m3d<true>(flo * sqrt_pi); }
         else lref = logref[f0 - 1];
         if (arg <= lref) continue;
       }

@@ -65,7 +65,8 @@ __device__ __forceinline__ float rcp_markstein(float d) {
 // e comes from the bits less those of the float after sqrt(1/2).  s is the correctly
 // rounded quotient: the product by the correctly rounded reciprocal, one correction by
 // the remainder (Markstein, as rcp_markstein); equal to the division at all 2^23
-// mantissas (an exhaustive comparison).
+// mantissas (an exhaustive comparison).  DIV: the division itself, the same bits.
+template <bool DIV = false>
 __device__ __forceinline__ float logf_m3d(float x) {
   int e = 0;
   if (__float_as_uint(x) - 0x00800000u >= 0x7f000000u) {   // not a normal positive number
@@ -77,8 +78,14 @@ __device__ __forceinline__ float logf_m3d(float x) {
   const int u = __float_as_int(x), k = (u - 0x3f3504f4) >> 23;
   e += k;
   const float f = __int_as_float(u - (k << 23)) - 1.0f;
-  const float d = 2.0f + f, rd = rcp_markstein(d), q0 = f * rd;
-  const float s = fmaf(fmaf(-q0, d, f), rd, q0);
+  const float d = 2.0f + f;
+  float s;
+  if (DIV) {
+    s = f / d;
+  } else {
+    const float rd = rcp_markstein(d), q0 = f * rd;
+    s = fmaf(fmaf(-q0, d, f), rd, q0);
+  }
   const float s2 = s * s;
   float p = fmaf(s2, 0.0909090936f, 0.111111112f);
   p = fmaf(s2, p, 0.142857143f);

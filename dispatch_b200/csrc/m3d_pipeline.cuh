@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(256) k_lte_opacity_units(AtmosDev A, GridArgs 
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int warps = blockDim.x >> 5;
   const int nf = G.nf;
-  const float lt = logf_m3d(G.tol / 0.5641895835f);
+  const float lt = logf_m3d<true>(G.tol / 0.5641895835f);
   float *s_x = smem + 2 * QLG_NTAB + (size_t)wid * 4 * nf;
   float *s_lr = s_x + nf, *s_chi = s_lr + nf, *s_eta = s_chi + nf;
   for (int cell = blockIdx.x * warps + wid; cell < A.ncell; cell += gridDim.x * warps) {
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(256) k_lte_opacity_units(AtmosDev A, GridArgs 
     for (int f = lane; f < nf; f += 32) {
       const float xh = point_xhat(chi_c, h_kT, nu[f]);
       s_x[f] = xh;
-      s_lr[f] = xh > 0.0f ? lt + logf_m3d(xh) : -FLT_MAX;
+      s_lr[f] = xh > 0.0f ? lt + logf_m3d<true>(xh) : -FLT_MAX;
       s_chi[f] = 0.0f;
       s_eta[f] = 0.0f;
     }
