@@ -484,7 +484,8 @@ __device__ __forceinline__ void deposit_adj(float (&chl)[NF], const float (&gch)
 //   dK/du = L^2 (cZH W' - (2 L P + bL)) - ln2 G gG,  P = cZH W + cL2,
 //   dK/dih = dK/du 2 u/ih + L (L (W dcZH + dcL2) + dbL) + G dgG,
 // FAR: W, W' and G the last node's at every point.  Points outside a partial window add
-// K = 0 and have their sensitivity left out.  The scalar form took some 24 instructions
+// K = 0, and neither their sensitivity nor their adjoint, which need not be finite,
+// enters the sums.  The scalar form took some 24 instructions
 // a point, this one 13.
 template <int NF, bool FULL, bool FAR>
 __device__ __forceinline__ void deposit_adj_x2(float (&chl)[NF], const float (&gch)[NF], const float2 *s_tab,
@@ -554,6 +555,7 @@ __device__ __forceinline__ void deposit_adj_x2(float (&chl)[NF], const float (&g
     const f32x2 t = fma2(NEG, fma2(add2(L, L), P, BL), cWd);
     const f32x2 dKu = fma2(mul2(L, L), t, gG);
     f32x2 dKi = fma2(dKu, mul2(u, R2IH), fma2(L, fma2(L, e, DBL), eg));
+    f32x2 gc = pk2(gch[2 * k], gch[2 * k + 1]);
     if (!FULL) {
       float ka, kb, ha, hb;
       up2(K, ka, kb);
@@ -561,12 +563,12 @@ __device__ __forceinline__ void deposit_adj_x2(float (&chl)[NF], const float (&g
       const bool ina = 2 * k + 1 >= fa && 2 * k + 1 <= fb, inb = 2 * k + 2 >= fa && 2 * k + 2 <= fb;
       K = pk2(ina ? ka : 0.0f, inb ? kb : 0.0f);
       dKi = pk2(ina ? ha : 0.0f, inb ? hb : 0.0f);
+      gc = pk2(ina ? gch[2 * k] : 0.0f, inb ? gch[2 * k + 1] : 0.0f);
     }
     float lo, hi;
     up2(add2(K, pk2(chl[2 * k], chl[2 * k + 1])), lo, hi);
     chl[2 * k] = lo;
     chl[2 * k + 1] = hi;
-    const f32x2 gc = pk2(gch[2 * k], gch[2 * k + 1]);
     G2 = fma2(gc, K, G2);
     H2 = fma2(gc, dKi, H2);
   }
