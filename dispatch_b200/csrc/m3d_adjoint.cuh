@@ -710,11 +710,12 @@ __global__ void __launch_bounds__(512, 1) k_opacity_adj(AtmosDev A, GridArgs G, 
           deposit_adj_x2<NF, true, false>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
         else
           deposit_adj_x2<NF, false, false>(chl, gch, s_tab, s_dW, cf, cd, x0, kfa, fa, fb, Gl, Hl);
-        // K is proportional to S = Rij D: dK/dD = K/D + dK/dih dih/dD, the first term's
-        // sum over the lines from gB
+        // K is proportional to S = Rij D: D dK/dD = K + dK/dih D dih/dD.  A line's two terms
+        // are added before they enter the sum: in a wing, which does not depend on D, they
+        // cancel
         gB += Gl;
         gE -= rec[l].lower_ev * Gl;
-        gD += Hl * dih_dD(a, qw.D);
+        gD += fmaf(Hl, dih_dD(a, qw.D) * qw.D, Gl);
         cg::coalesced_group grp = cg::coalesced_threads();
         const float tot = cg::reduce(grp, Gl, cg::plus<float>());
         if (grp.thread_rank() == 0) atomicAdd(&s_gp[sp * nline_max + l], tot);
@@ -722,8 +723,8 @@ __global__ void __launch_bounds__(512, 1) k_opacity_adj(AtmosDev A, GridArgs G, 
       if (live) {
         const size_t o = (size_t)ncell * ((size_t)ray * A.nspecies + sp) + cs;
         p_lnbase[o] = gB;
-        // D = sdl / idf
-        p_idf[o] = (gB / qw.D + gD) * (-qw.D / idf);
+        // D = sdl / idf: dD/didf = -D / idf, and gD holds D dL/dD
+        p_idf[o] = -(gD / idf);
       }
     }
     if (live) p_ekt[rc] = gE;
