@@ -9,6 +9,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -144,6 +145,18 @@ int scratch(int slot, size_t bytes, void **out) {
   }
   *out = g_ctx.scratch[slot];
   return M3D_OK;
+}
+
+// gives slots back, before a second attempt with less
+void scratch_release(std::initializer_list<int> slots) {
+  cudaGetLastError();   // the allocation that failed
+  cudaStreamSynchronize(g_ctx.stream);
+  for (int k : slots) {
+    if (k >= (int)g_ctx.scratch.size() || !g_ctx.scratch[k]) continue;
+    cudaFree(g_ctx.scratch[k]);
+    g_ctx.scratch[k] = nullptr;
+    g_ctx.scratch_bytes[k] = 0;
+  }
 }
 
 // Host-pointer staging for one call: device copies of the arguments, copied
@@ -1568,14 +1581,7 @@ int lte_synthesis_impl(const m3d_atmos_t *atm, int nwin, int nf_win, const doubl
   const size_t esz = fp64 ? sizeof(double) : sizeof(float);
   int group = nwin > 1 ? nray : (in.reach ? 1 : rays_per_launch(in.ncell, nf, nray, esz));
   group = std::min(group, 32768);  // the grid limit of the launches below
-  void *dchi, *dS, *dtop;
-  if (nwin == 1 && group > 1 &&
-      (scratch(7, esz * plane * nz * group, &dchi) != M3D_OK || scratch(8, esz * plane * nz * group, &dS) != M3D_OK)) {
-    cudaGetLastError();
-    group = 1;
-  }
-  TRY(scratch(7, esz * plane * nz * group, &dchi));
-  TRY(scratch(8, esz * plane * nz * group, &dS));
+  void *dtop;
   void *dtop_user = nullptr;
   if (i_top) {
     if (fp64) { double *p; TRY(st.map((double *)i_top, plane * nray, false, true, &p)); dtop_user = p; }
@@ -1608,8 +1614,6 @@ int lte_synthesis_impl(const m3d_atmos_t *atm, int nwin, int nf_win, const doubl
   // partial sums of the intensity reduction: blocks of 8 columns, at most 148 of them
   // (a part without columns would add a zero)
   const int kParts = (int)std::min<size_t>(148, (ncol + 7) / 8);
-  void *dpart;
-  TRY(scratch(12, sizeof(double) * kParts * nf * group, &dpart));
 
   // FP64 plain path buffers
   void *dwork = nullptr, *dmem = nullptr;
@@ -1619,6 +1623,20 @@ int lte_synthesis_impl(const m3d_atmos_t *atm, int nwin, int nf_win, const doubl
     TRY(scratch(10, sizeof(double) * plane * (maxn + 2) * 3, &dwork));
     TRY(scratch(11, sizeof(double) * plane * 3, &dmem));
   }
+
+  // the group's arrays last: where they can't be had, one ray's, and what the group's
+  // took is given back first
+  void *dchi, *dS, *dpart;
+  auto group_arrays = [&](size_t g) {
+    TRY(scratch(7, esz * plane * nz * g, &dchi));
+    TRY(scratch(8, esz * plane * nz * g, &dS));
+    return scratch(12, sizeof(double) * kParts * nf * g, &dpart);
+  };
+  if (nwin == 1 && group > 1 && group_arrays(group) != M3D_OK) {
+    scratch_release({7, 8, 12});
+    group = 1;
+  }
+  TRY(group_arrays(group));
 
   for (int r0 = 0; r0 < nray; r0 += group) {
     const int nr = std::min(group, nray - r0);
