@@ -1,0 +1,39 @@
+"""Point counts on both sides of the line that parts the forms of the model atom's line
+opacities, the lines' constants formed ahead or at every point (2 Mi points): bit for bit
+against the oracle."""
+import numpy as np
+import pytest
+
+from dispatch_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _cells(ncell, transitions, nper, seed=11):
+    atom, inp = synth.se_config("small", ncell=ncell)
+    win = synth.atom_window(atom, nper=nper, transitions=[k if k >= 0 else atom["nline"] - k - 1 for k in transitions])
+    rng = np.random.default_rng(seed)
+    c = {"b": inp["b"], "nstar": inp["nstar"], "pop_ratio": np.ones(ncell), "e_kT": inp["e_kT"],
+         "inv_df": (1.8e5 * (1 + 0.1 * rng.standard_normal(ncell))).astype(np.float32),
+         "vproj": (1e-5 * rng.standard_normal(ncell)).astype(np.float32),
+         "adamp": rng.uniform(1e-3, 0.1, (max(win["nline"], 1), ncell)).astype(np.float32)}
+    return win, c, rng
+
+
+@pytest.mark.parametrize("ncell", [3, 10485, 10486])
+@pytest.mark.parametrize("lte", [False, True])
+def test_bb_opacity_points(m3d, oracle, ncell, lte):
+    from dispatch_b200 import nlte as gn
+    from oracle import nlte as nl
+    win, c, rng = _cells(ncell, range(0, 40, 5), 25)
+    assert win["nf"] == 200
+    x, e = (1e-8 * (1 + rng.random((ncell, 200), np.float32)) for _ in range(2))
+    res = []
+    for mod in (nl, gn):
+        xh, eh, sp = x.copy(), e.copy(), gn.new_split(ncell, 200)
+        mod.bb_opacity(win, c["b"], c["nstar"], c["pop_ratio"], c["e_kT"], c["inv_df"], c["vproj"], c["adamp"], xh,
+                       eh, lte=lte, split=sp)
+        res.append((xh, eh, *sp.values()))
+    for o, g in zip(*res):
+        np.testing.assert_array_equal(g, o)
+    assert not np.array_equal(res[0][0], x)
