@@ -1,6 +1,7 @@
-"""Calls where the device memory is nearly full.  The rays that share a launch take
-more memory than a call needs: where it can't be had the call runs with less and gives the
-same results, at every amount that is left.  Each runs in a thread, with a library context of
+"""Calls where the device memory is nearly full.  The rays that share a launch, the lines'
+constants of the NLTE opacity and a column plan's windows side by side take more memory
+than a call needs: where it can't be had the call runs with less and gives the same
+results, at every amount that is left.  Each runs in a thread, with a library context of
 its own that holds nothing yet."""
 import threading
 
@@ -95,3 +96,31 @@ def test_gradient_rays_one_by_one(m3d):
             assert torch.equal(got[k], want[k]), (leave, k)
         # the lines' sums over the cells in any order
         np.testing.assert_allclose(got["gpref"], want["gpref"], rtol=1e-4, atol=1e-6 * float(want["gpref"].abs().max()))
+
+
+def test_line_constants_at_every_point(m3d):
+    """106000 cells x 20 lines: 64 MB of the lines' constants where there is room for them,
+    formed at every point where there is not."""
+    import torch
+    from dispatch_b200 import nlte
+    nc = 106000
+    atom, inp = synth.se_config("small", ncell=nc)
+    win = synth.atom_window(atom, nper=5, transitions=list(range(20)))
+    rng = np.random.default_rng(3)
+    s = {"b": inp["b"], "nstar": inp["nstar"], "pop_ratio": np.ones(nc), "e_kT": inp["e_kT"],
+         "inv_df": (1.8e5 * (1 + 0.1 * rng.standard_normal(nc))).astype(np.float32),
+         "vproj": (1e-5 * rng.standard_normal(nc)).astype(np.float32),
+         "adamp": rng.uniform(1e-3, 0.1, (win["nline"], nc)).astype(np.float32)}
+    up = [torch.as_tensor(np.ascontiguousarray(v), device="cuda") for v in s.values()]
+    base = [torch.full((nc, win["nf"]), 1e-9, device="cuda") for _ in range(2)]
+
+    def run(x, e):
+        nlte.bb_opacity(win, *up, x, e)
+        m3d.synchronize()
+
+    want, got = [b.clone() for b in base], [b.clone() for b in base]
+    _in_thread(run, *want)
+    with _Full(40 * MB):
+        _in_thread(run, *got)
+    for g, w, b in zip(got, want, base):
+        assert torch.equal(g, w) and not torch.equal(g, b)
