@@ -546,29 +546,30 @@ k_bb_rates(NlWinDev W, NlRateOpts O, int ncell, const double *__restrict__ b,
   }
 }
 
-// One warp per (continuum, kBbCells consecutive cells): a cell's terms with the lanes
-// along f, then one sum a lane (three sums of eight cells) in ascending f.  A warp per
-// cell ran its sums on three of its lanes: 0.15 -> 0.10 ms for 81000 cells and three
-// continua of 25 frequencies.
+// One warp per (continuum, C consecutive cells): a cell's terms with the lanes along f,
+// then one sum a lane (three sums of C cells) in ascending f.  C = 8 where the tiles fill
+// the GPU (a warp per cell runs its sums on three of its lanes: 0.15 -> 0.10 ms for 81000
+// cells and three continua of 25 frequencies), C = 1 where they do not.
+template <int C>
 __global__ void __launch_bounds__(kRateWarps * 32)
 k_bf_rates(NlWinDev W, int ncell, int precond, const double *__restrict__ b,
            const double *__restrict__ nstar, const double *__restrict__ e_kT,
            const float *__restrict__ twohnu3_c2, const float *__restrict__ Jnu,
            const float *__restrict__ PsiJ, const float *__restrict__ beta,
            float *__restrict__ gamma_ij, float *__restrict__ gamma_ji) {
-  __shared__ float sh[kRateWarps][3][kBbCells][33];
+  __shared__ float sh[kRateWarps][3][C][33];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  float (*T)[kBbCells][33] = sh[wib];
+  float (*T)[C][33] = sh[wib];
   const size_t nf = (size_t)W.nf;
-  const size_t n = (size_t)((ncell + kBbCells - 1) / kBbCells) * W.ncont;
+  const size_t n = (size_t)((ncell + C - 1) / C) * W.ncont;
   const size_t stride = (size_t)gridDim.x * kRateWarps;
   for (size_t kk = (size_t)blockIdx.x * kRateWarps + wib; kk < n; kk += stride) {
-    const int j = (int)(kk % W.ncont), c0 = (int)(kk / W.ncont) * kBbCells;
+    const int j = (int)(kk % W.ncont), c0 = (int)(kk / W.ncont) * C;
     if (W.cactive && !W.cactive[j]) continue;
     const int li = W.ci[j], lj = W.cj[j], fs = W.cblue[j], fe = W.cred[j], off = W.coff[j];
-    const int ncl = min(kBbCells, ncell - c0);
-    const int ck = c0 + lane % kBbCells;      // the cell whose sum this lane forms
-    const bool mine = lane < 3 * kBbCells && lane % kBbCells < ncl &&
+    const int ncl = min(C, ncell - c0);
+    const int ck = c0 + lane % C;      // the cell whose sum this lane forms
+    const bool mine = lane < 3 * C && lane % C < ncl &&
                       !((W.ev[lj] - W.ev[li]) * e_kT[ck] > W.cut_x);
     if (!__any_sync(0xffffffffu, mine)) continue;
     // sum_abs, sum_ems, sum_pre
@@ -600,15 +601,15 @@ k_bf_rates(NlWinDev W, int ncell, int precond, const double *__restrict__ b,
       __syncwarp();
       if (mine) {
         const int cnt = min(32, fe - f0 + 1);
-        const float *row = T[lane / kBbCells][lane % kBbCells];
+        const float *row = T[lane / C][lane % C];
 #pragma unroll 8
         for (int q = 0; q < cnt; q++) acc = acc + row[q];
       }
       __syncwarp();
     }
-    const float sum_ems = __shfl_sync(0xffffffffu, acc, (lane + kBbCells) & 31);
-    const float sum_pre = __shfl_sync(0xffffffffu, acc, (lane + 2 * kBbCells) & 31);
-    if (mine && lane < kBbCells) {
+    const float sum_ems = __shfl_sync(0xffffffffu, acc, (lane + C) & 31);
+    const float sum_pre = __shfl_sync(0xffffffffu, acc, (lane + 2 * C) & 31);
+    if (mine && lane < C) {
       float g_ij = acc, g_ji = sum_ems;
       if (precond) {
         const double nsi = nstar[(size_t)ck + (size_t)ncell * li];

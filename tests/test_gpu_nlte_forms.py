@@ -1,6 +1,7 @@
-"""Point counts on both sides of the line that parts the forms of the model atom's line
-opacities, the lines' constants formed ahead or at every point (2 Mi points): bit for bit
-against the oracle."""
+"""Cell counts on both sides of the lines that part the forms of the model atom's kernels:
+the continuum rates with eight cells or one a warp (two blocks of tiles an SM), the line
+opacities with the lines' constants formed ahead or at every point (2 Mi points); bit for
+bit against the oracle."""
 import numpy as np
 import pytest
 
@@ -18,6 +19,27 @@ def _cells(ncell, transitions, nper, seed=11):
          "vproj": (1e-5 * rng.standard_normal(ncell)).astype(np.float32),
          "adamp": rng.uniform(1e-3, 0.1, (max(win["nline"], 1), ncell)).astype(np.float32)}
     return win, c, rng
+
+
+@pytest.mark.parametrize("ncell,ncont", [(1, 1), (9, 3), (18936, 1), (18937, 1), (18943, 1), (944, 20),
+                                         (945, 20), (1184, 16), (2369, 8)])
+@pytest.mark.parametrize("precond", [True, False])
+@pytest.mark.parametrize("cut_x", [70.0, 15.0])
+def test_bf_rates_tiles(m3d, oracle, ncell, ncont, precond, cut_x):
+    from dispatch_b200 import nlte as gn
+    from oracle import nlte as nl
+    win, c, rng = _cells(ncell, [-1 - k for k in range(ncont)], 37)
+    win["cut_x"] = cut_x            # 15: some cells leave the transition out
+    assert win["ncont"] == ncont and win["nline"] == 0
+    J, P = (rng.random((ncell, win["nf"])).astype(np.float32) for _ in range(2))
+    beta = rng.uniform(1e-3, 0.6, (ncell, win["nf"])).astype(np.float32)
+    res = []
+    for mod in (nl, gn):
+        g = [np.full((ncont, ncell), 0.25, np.float32) for _ in range(2)]
+        mod.bf_rates(win, c["b"], c["nstar"], c["e_kT"], J, P, beta, *g, preconditioning=precond)
+        res.append(g)
+    for o, g in zip(*res):
+        np.testing.assert_array_equal(g, o)
 
 
 @pytest.mark.parametrize("ncell", [3, 10485, 10486])
