@@ -25,6 +25,7 @@ namespace m3d {
 
 struct NlWinDev {
   int nf, nline, ncont;
+  int line_pts;        // the lines' mean number of points
   const int *li, *lj, *lntrans, *lindex, *lblue, *lred, *loff;
   const float *q;
   const double *wnu, *wq, *Bij, *Aij, *lower_ev, *grad, *gw1, *gw2, *gstk;
@@ -359,15 +360,16 @@ constexpr int kRateWarps = 8;
 // sectors their windows share (and those a window straddles) are read from DRAM
 // once and from L2 after.  Each (line, cell) has one writer, so the order changes
 // no sum.
-// 8 cells a tile (17 KB of shared terms a block) and 48 registers give 10 blocks (40
-// warps) per SM, which hides the loads' latency better than 16-cell tiles at 6 blocks
-// (the 120^3 window's sweep 748 -> 711 ms at 8) or 8-cell ones at 8: 0.43 -> 0.41 ms a
-// direction of 48^3 cells, 8 lines and 250 frequencies, in spite of 56 bytes spilled.  Staging
-// the twelve arrays with asynchronous copies (16 warps) took 0.63 ms, two and four
-// cells' loads together 0.48-0.53, the lines' constants from a pass of their own 0.43.
+// 8 cells a tile, 18 KB of shared terms a block; 10 blocks (40 warps) per SM with 48
+// registers and 56 bytes spilled, or 8 with 64.  The loads' latency is hidden better than
+// with 16-cell tiles at 6 blocks (the 120^3 window's sweep 748 -> 711 ms at 8).  Staging
+// the twelve arrays with asynchronous copies (16 warps) took 0.63 ms a direction of 48^3
+// cells, 8 lines and 250 frequencies, two and four cells' loads together 0.48-0.53, the
+// lines' constants from a pass of their own 0.43, this form 0.41.
 constexpr int kBbWarps = 4, kBbCells = 8;
 
-__global__ void __launch_bounds__(kBbWarps * 32, 10)
+template <int MINB>
+__global__ void __launch_bounds__(kBbWarps * 32, MINB)
 k_bb_rates(NlWinDev W, NlRateOpts O, int ncell, const double *__restrict__ b,
            const double *__restrict__ nstar, const double *__restrict__ pop_ratio,
            const double *__restrict__ e_kT, const float *__restrict__ inv_df,

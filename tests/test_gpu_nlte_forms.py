@@ -1,7 +1,7 @@
 """Cell counts on both sides of the lines that part the forms of the model atom's kernels:
 the continuum rates with eight cells or one a warp (two blocks of tiles an SM), the line
-opacities with the lines' constants formed ahead or at every point (2 Mi points); bit for
-bit against the oracle."""
+opacities with the lines' constants formed ahead or at every point (2 Mi points), the line
+rates by their lines' points; bit for bit against the oracle."""
 import numpy as np
 import pytest
 
@@ -59,3 +59,34 @@ def test_bb_opacity_points(m3d, oracle, ncell, lte):
     for o, g in zip(*res):
         np.testing.assert_array_equal(g, o)
     assert not np.array_equal(res[0][0], x)
+
+
+@pytest.mark.parametrize("nper", [25, 32, 33, 70])
+@pytest.mark.parametrize("split_rates", [True, False])
+@pytest.mark.parametrize("precond", [True, False])
+def test_bb_rates_line_points(m3d, oracle, nper, split_rates, precond):
+    """The line rates with ten and with eight blocks an SM: lines of up to and beyond one
+    round of the lanes."""
+    from dispatch_b200 import nlte as gn
+    from oracle import nlte as nl
+    n = 61
+    win, c, rng = _cells(n, range(0, 40, 5), nper)
+    nf = win["nf"]
+    f32 = lambda lo, hi: rng.uniform(lo, hi, (n, nf)).astype(np.float32)
+    beta = f32(1e-3, 0.6)
+    ids = lambda: rng.integers(0, 12, (n, nf)).astype(np.int32)
+    split = {"opac_L": f32(0, 1), "opac_R": f32(0, 1), "id": ids(), "chi_L": f32(0, 1), "chi_R": f32(0, 1),
+             "chi_id": ids()}
+    kw = dict(work1=f32(0.1, 1), psi=f32(0, 1), irem=f32(0, 1), escape=f32(0, 1), split=split,
+              split_rates=split_rates, preconditioning=precond, wmu=0.3)
+    kw["psi"][rng.random((n, nf)) < 0.05] = 0.0
+    inu, Bnu = f32(0, 1), beta / (1 - beta)
+    res = []
+    for mod in (nl, gn):
+        g = [np.full((win["nline"], n), 0.25, np.float32) for _ in range(2)]
+        mod.bb_rates(win, c["b"], c["nstar"], c["pop_ratio"], c["e_kT"], c["inv_df"], c["vproj"], c["adamp"], inu,
+                     beta, Bnu, *g, **kw)
+        res.append(g)
+    for o, g in zip(*res):
+        np.testing.assert_array_equal(g, o)
+    assert np.abs(res[0][0]).max() > 0.25
