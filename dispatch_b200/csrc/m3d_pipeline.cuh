@@ -306,11 +306,14 @@ __device__ __forceinline__ void deposit_window_mk(float (&chl)[NF], const float2
   }
 }
 
-// lround of a double (half away from zero) for |x| < 2^31: floor(|x| + 0.5) with the
+// lround of a double (half away from zero) for |x| <= 2^29: floor(|x| + 0.5) with the
 // sum rounded toward zero, which never reaches the next integer below the exact sum
 // (an integer below 2^53 is representable), so it is exact; the conversion truncates.
+// Larger |x|, as an infinite velocity gives, stay at 2^29: a line's place and its
+// window's reach are added and counted from 1, and a sum past 2^31 is undefined, so that
+// a place clamped to the window afterwards was not sure to lie in it.
 __device__ __forceinline__ int lround_d(double x) {
-  const int m = __double2int_rz(__dadd_rz(fabs(x), 0.5));
+  const int m = min(__double2int_rz(__dadd_rz(fabs(x), 0.5)), 1 << 29);
   return x < 0.0 ? -m : m;
 }
 
