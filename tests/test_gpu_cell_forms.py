@@ -11,7 +11,7 @@ from dispatch_b200 import synth
 pytestmark = pytest.mark.gpu
 
 SMS = 148
-CONT = SMS * 64                  # the continuum's line
+CONT = SMS * 32 + 1              # the continuum's line
 BG, LL = SMS * 3 * 8 * 8, SMS * 2 * 8 * 4 * 6
 
 
