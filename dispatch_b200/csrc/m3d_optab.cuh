@@ -330,12 +330,7 @@ __global__ void __launch_bounds__(32 * kOptabWarps, 2) k_optab_sample_ll(OptabDe
 // ---- a cell a warp ----------------------------------------------------------------
 // For cell counts that give the grouped kernels less than the warps they need: the
 // neighbours' turns in a warp then only add up.  64 registers at 4 blocks an SM, the
-// corners read pair by pair.  The cells are called small below a full round of the
-// grouped kernel's warps on the GPU (28416 cells), for the line list below six (56832),
-// whose last round of longer turns weighs more.  256 frequencies, a cell a warp against
-// groups: 512 cells 44 and 58 us, for the line list 79 and 95; 4096 cells 41 / 48 and
-// 69 / 83; 13824 57 / 56 and 106 / 118; 32768 86 / 78 and 196 / 203; 64000 140 / 108 and
-// 345 / 325.
+// corners read pair by pair.  Where the line lies: optab_grouped, optab_grouped_ll.
 
 // collapse of a query between the nodes at and at + 1
 __device__ __forceinline__ float optab_collapse_at(const float4 *t, long long at, int sit, long long sje,

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 SMS = 148
 CONT = SMS * 32 + 1              # the continuum's line
-BG, LL = SMS * 3 * 8 * 8, SMS * 2 * 8 * 4 * 6
+BG, ROUND = SMS * 8 * 8, SMS * 2 * 8 * 4      # the samplers': a block of groups an SM, a round
 
 
 def _exact_comps(comps):
@@ -62,7 +62,9 @@ def test_continuum_table_rows(m3d, oracle, ncell, nnu, ncomp):
     _continuum(comps, lam, nu, cells, ncell)
 
 
-@pytest.mark.parametrize("ncell", [BG - 1, BG, BG + 1, BG + 7, LL - 1, LL, LL + 1, LL + 3])
+@pytest.mark.parametrize("ncell", [ROUND * 19 // 20, ROUND * 19 // 20 + 1, BG - 1, BG, BG + 1, BG + 7,
+                                   2 * ROUND * 19 // 20, 2 * ROUND * 19 // 20 + 1, 2 * ROUND + 1,
+                                   5 * ROUND, 5 * ROUND + 1, 5 * ROUND + 3])
 def test_table_counts(m3d, oracle, ncell):
     from dispatch_b200.optab import SampleOptab
     from oracle import optab
