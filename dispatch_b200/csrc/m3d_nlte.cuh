@@ -25,7 +25,7 @@ namespace m3d {
 
 struct NlWinDev {
   int nf, nline, ncont;
-  int line_pts;        // the lines' mean number of points
+  int line_pts, cont_pts;   // the lines' and the continua's mean number of points
   const int *li, *lj, *lntrans, *lindex, *lblue, *lred, *loff;
   const float *q;
   const double *wnu, *wq, *Bij, *Aij, *lower_ev, *grad, *gw1, *gw2, *gstk;

@@ -1,7 +1,7 @@
 """Cell counts on both sides of the lines that part the forms of the model atom's kernels:
-the continuum rates with eight cells or one a warp (two blocks of tiles an SM), the line
-opacities with the lines' constants formed ahead or at every point (2 Mi points), the line
-rates by their lines' points; bit for bit against the oracle."""
+the continuum rates with eight cells or one a warp (a block of tiles an SM, two for long
+continua), the line opacities with the lines' constants formed ahead or at every point (2
+Mi points), the line rates by their lines' points; bit for bit against the oracle."""
 import numpy as np
 import pytest
 
@@ -21,14 +21,15 @@ def _cells(ncell, transitions, nper, seed=11):
     return win, c, rng
 
 
-@pytest.mark.parametrize("ncell,ncont", [(1, 1), (9, 3), (18936, 1), (18937, 1), (18943, 1), (944, 20),
-                                         (945, 20), (1184, 16), (2369, 8)])
+@pytest.mark.parametrize("ncell,ncont,nper", [(1, 1, 37), (9, 3, 37), (9464, 1, 37), (9465, 1, 37), (9471, 1, 37),
+                                              (472, 20, 5), (473, 20, 5), (592, 16, 5), (1185, 8, 5),
+                                              (944, 20, 30), (945, 20, 30), (1184, 16, 30)])
 @pytest.mark.parametrize("precond", [True, False])
 @pytest.mark.parametrize("cut_x", [70.0, 15.0])
-def test_bf_rates_tiles(m3d, oracle, ncell, ncont, precond, cut_x):
+def test_bf_rates_tiles(m3d, oracle, ncell, ncont, nper, precond, cut_x):
     from dispatch_b200 import nlte as gn
     from oracle import nlte as nl
-    win, c, rng = _cells(ncell, [-1 - k for k in range(ncont)], 37)
+    win, c, rng = _cells(ncell, [-1 - k for k in range(ncont)], nper)
     win["cut_x"] = cut_x            # 15: some cells leave the transition out
     assert win["ncont"] == ncont and win["nline"] == 0
     J, P = (rng.random((ncell, win["nf"])).astype(np.float32) for _ in range(2))
