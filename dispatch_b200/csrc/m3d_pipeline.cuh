@@ -99,8 +99,8 @@ __device__ __forceinline__ float point_xhat(float chi_c, float h_kT, double nu) 
   return chi_c + chi_c * Bnu;
 }
 
-// One warp per cell, for the windows and line lists that the lane kernel below does not
-// take: fewer than 8 frequencies, or reach_in with other than 32.
+// One warp per cell, for what the lane kernel below does not take: fewer than 8
+// frequencies, one ray of few cells, or reach_in with other than 32 frequencies.
 // Shared memory: the two QLG tables, then per warp xhat, logref, chi_l, eta_l (nf each)
 __global__ void __launch_bounds__(256) k_lte_opacity_units(AtmosDev A, GridArgs G, const double *nu, double v0,
                                                            double v1, double v2, float *chi_out, float *S_out,
@@ -317,8 +317,10 @@ __device__ __forceinline__ int lround_d(double x) {
   return x < 0.0 ? -m : m;
 }
 
-// lroundf of v >= 0, the same way in float (above 2^23 v is an integer and stays)
+// lround of v >= 0 the same way, in float (above 2^23 v is an integer and stays) and in
+// double below 2^31
 __device__ __forceinline__ int lround_pos(float v) { return __float2int_rz(__fadd_rz(v, 0.5f)); }
+__device__ __forceinline__ int lround_pos(double v) { return __double2int_rz(__dadd_rz(v, 0.5)); }
 
 template <int NF>
 __device__ __forceinline__ float pick(const float (&a)[NF], int i) {
@@ -736,7 +738,7 @@ __global__ void __launch_bounds__(512, 1) k_lte_opacity_units_f64(AtmosDev A, Gr
         const double x1 = (G.llam[f0 - 1] - llc) * G.inv_dllam;
         const QlgCoef64 cf = qlg_setup64(a, D, SQ, S);
         const double hw = qlg_halfwidth64(D2, a, S, refl, arg - lref);
-        const int noff = lround_d(fmin(hw, (double)(nf + abs(ic))));
+        const int noff = lround_pos(fmin(hw, (double)(nf + abs(ic))));
         const int fa = ic - noff > 1 ? ic - noff : 1;
         const int fb = ic + noff < nf ? ic + noff : nf;
         const int ga = max(fa, o + 1), gb = min(fb, o + nl);
