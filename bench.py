@@ -162,8 +162,8 @@ def _peaks():
 #  k_quad_rot_column2: DRAM bytes per cell and frequency of a launch (28,360,192 B read
 #    for 110,592 cells x 32 frequencies), against 8 B algorithmic (chi and Snu once).
 #  k_lte_opacity_units_lane<32>: warp instructions per (cell, line), the mean over the
-#    8 timed windows x 13 rays, 16 launches (66,867,942,996 for 110,592 cells x
-#    500 lines each; 11.1-12.2 by window as their line loads differ), which
+#    8 timed windows x 13 rays, 16 launches (67,047,654,996 for 110,592 cells x
+#    500 lines each; 11.1-12.3 by window as their line loads differ), which
 #    scales a full launch's count by its cells and lines; DRAM bytes per cell: 49.9 B
 #    read (measured, window 0) plus the chi and
 #    Snu it writes, 8 B per frequency (the small case's 28 MB of output stayed in L2,
@@ -172,7 +172,7 @@ NCU_SWEEP_DRAM_BYTES_PER_CELL_FREQ = 8.013
 #  k_quad_rot_column2: warp instructions per (cell, frequency), the mean over the same
 #    windows and rays (2,349,966,639 for 110,592 cells x 32 frequencies each)
 NCU_SWEEP_WARP_INST_PER_CELL_FREQ = 2349966639 / (104 * 110592 * 32)
-NCU_OPACITY_WARP_INST_PER_CELL_LINE = 66867942996 / (104 * 110592 * 500)
+NCU_OPACITY_WARP_INST_PER_CELL_LINE = 67047654996 / (104 * 110592 * 500)
 NCU_OPACITY_DRAM_READ_BYTES_PER_CELL = 5516032 / 110592
 #  k_continuum: warp instructions per cell of a launch of the continuum case (250
 #    frequencies, fourteen components; 814,461,731 for 110,592 cells)

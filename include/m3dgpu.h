@@ -927,7 +927,9 @@ typedef struct m3d_col_plan m3d_col_plan_t;
 /* A plan for one model atom over its frequency windows: the windows' tables are
  * staged once (win_nu float64, win_twohnu3_c2 float32 per window, host or device;
  * win_adamp the window lines' damping (nline, ncell), device), and the plan owns
- * work arrays sized for the widest window.  A window whose every frequency lies in
+ * work arrays sized for the widest window, one set for each of the windows that are
+ * swept side by side (within 8 GiB and, beyond the first set, a quarter of the memory
+ * free at the call).  A window whose every frequency lies in
  * at most 4 line windows is swept by one fused kernel per hemisphere (line opacity,
  * transfer units, the column solve, J/PsiJ and the line rates of a column in one
  * CTA); the others, and every window with M3D_COL_PERPOINT, by the per-point
