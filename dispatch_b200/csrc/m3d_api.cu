@@ -1190,12 +1190,16 @@ namespace {
 
 int sm_count();   // m3d_stateq_api.inc
 
-// 72 KB of tables in shared memory for a lane kernel
-int lane_attr(const void *kernel) {
-  CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(2 * QLG_NTAB * sizeof(float))));
+// The dynamic shared memory a kernel may have.  The limit belongs to the kernel, not to
+// the calling thread: every caller sets the largest that any call can want, so that none
+// lowers it between another thread's setting and its launch.
+int smem_limit(const void *kernel, size_t most) {
+  CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   return M3D_OK;
 }
+
+// 72 KB of tables in shared memory for a lane kernel
+int lane_attr(const void *kernel) { return smem_limit(kernel, 2 * QLG_NTAB * sizeof(float)); }
 
 // a zeroed counter of the units handed out by the next launch
 int unit_counter(int **next) {
@@ -1381,12 +1385,7 @@ int launch_opacity(SynthIn &in, const double *v, const double *d_vr, int nray, b
   const bool lone = nray == 1 && nf != 32 && nf <= 128 && ncell <= (size_t)16 * sm_count();
   if (lf.NF == 0 || lone || (in.reach && nf != 32)) {
     const size_t smem = (2 * QLG_NTAB + (size_t)warps * 4 * nf) * sizeof(float);
-    thread_local size_t attr = 0;
-    if (attr < smem) {
-      CUDA_TRY(cudaFuncSetAttribute((const void *)k_lte_opacity_units, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-      attr = smem;
-    }
+    TRY(smem_limit((const void *)k_lte_opacity_units, (2 * QLG_NTAB + (size_t)warps * 4 * 1024) * sizeof(float)));
     const int grid = (int)std::min<size_t>((ncell + warps - 1) / warps, 148 * 16);
     for (int r = 0; r < nray; r++)
       LAUNCH_S(M3D_STAGE_OPACITY, k_lte_opacity_units, grid, block, smem, in.A, in.G, in.dnu, v[3 * r], v[3 * r + 1],
